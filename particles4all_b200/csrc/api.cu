@@ -291,6 +291,7 @@ void pack_params(p4a_sim* s, double dt) {
   F.skinH2 = (float)((h + kSkin * h) * (h + kSkin * h));
   F.skinHalf = (float)((kSkin * h - 1e-4 * h) * 0.5);
   F.volSpiky = F.volume * F.spikyGrad;
+  F.pairMath = pair_math_ranges(F);
 }
 
 uint32_t next_epoch(p4a_sim* s) {
@@ -321,9 +322,13 @@ int upload_boundary(p4a_sim* s) {
   const int nb = hb.count;
   if ((rc = dalloc(s, s->boundaryAllocs, &s->d.bpos, (size_t)std::max(1, nb)))) return rc;
   if ((rc = dalloc(s, s->boundaryAllocs, &s->d.bpsi, (size_t)std::max(1, nb)))) return rc;
+  if ((rc = dalloc(s, s->boundaryAllocs, &s->d.bsample, (size_t)std::max(1, nb)))) return rc;
   if ((rc = dalloc(s, s->boundaryAllocs, &s->d.bcellStart, (size_t)s->nCells + 2))) return rc;
+  std::vector<float> sample(hb.pos);
+  for (int k = 0; k < nb; k++) sample[(size_t)k * 4 + 3] = hb.psi[k];
   CUDA_TRY(s, cudaMemcpyAsync(s->d.bpos, hb.pos.data(), hb.pos.size() * 4, cudaMemcpyHostToDevice, s->stream));
   CUDA_TRY(s, cudaMemcpyAsync(s->d.bpsi, hb.psi.data(), hb.psi.size() * 4, cudaMemcpyHostToDevice, s->stream));
+  CUDA_TRY(s, cudaMemcpyAsync(s->d.bsample, sample.data(), sample.size() * 4, cudaMemcpyHostToDevice, s->stream));
   CUDA_TRY(s, cudaMemcpyAsync(s->d.bcellStart, hb.cellStart.data(), hb.cellStart.size() * 4,
                               cudaMemcpyHostToDevice, s->stream));
   CUDA_TRY(s, cudaStreamSynchronize(s->stream));  // host vectors go out of scope

@@ -122,6 +122,7 @@ void pack(BScene& s, double dt, int slot) {
   F.skinH2 = (float)((h + kSkin * h) * (h + kSkin * h));
   F.skinHalf = (float)((kSkin * h - 1e-4 * h) * 0.5);
   F.volSpiky = F.volume * F.spikyGrad;
+  F.pairMath = pair_math_ranges(F);
 }
 
 // Kinds of the launches of a frame, in the order a substep issues them.
@@ -485,7 +486,6 @@ int prepare_scene(const p4a_params& params, HostScene& sc, int pourBudget, Prepa
   ps.oPhase = o; o = a16(o + n16);
   ps.oRest = o; o = a16(o + n16);
   ps.oBpos = o; o = a16(o + ps.hb.pos.size() * 4);
-  ps.oBpsi = o; o = a16(o + ps.hb.psi.size() * 4);
   ps.oBcs = o; o = a16(o + ps.hb.cellStart.size() * 4);
   ps.oInfo = o; o = a16(o + (size_t)ps.nb1 * 16);
   ps.oCentre = o; o = a16(o + (size_t)ps.nb1 * 16);
@@ -507,7 +507,8 @@ void write_blob(const PreparedScene& ps, unsigned char* blob) {
     std::memcpy(blob + ps.oRest, sc.rest.data(), n16);
   }
   std::memcpy(blob + ps.oBpos, ps.hb.pos.data(), ps.hb.pos.size() * 4);
-  std::memcpy(blob + ps.oBpsi, ps.hb.psi.data(), ps.hb.psi.size() * 4);
+  float* sample = reinterpret_cast<float*>(blob + ps.oBpos);
+  for (int k = 0; k < ps.hb.count; k++) sample[(size_t)k * 4 + 3] = ps.hb.psi[k];
   std::memcpy(blob + ps.oBcs, ps.hb.cellStart.data(), ps.hb.cellStart.size() * 4);
   // bodies (src/sim.js:129-161); bodyStart relative to the scene's list range
   float* info = reinterpret_cast<float*>(blob + ps.oInfo);
@@ -573,8 +574,7 @@ int place_scene(p4a_batch* b, PreparedScene& ps, unsigned char* blob, cudaStream
     BTRY(b, cudaMemcpyAsync(d.rest[0] + po, blob + ps.oRest, nb, cudaMemcpyHostToDevice, st));
   }
   // boundary samples and their cellStart in arena indices
-  BTRY(b, cudaMemcpyAsync(d.bpos + s.bound.off, blob + ps.oBpos, ps.hb.pos.size() * 4, cudaMemcpyHostToDevice, st));
-  BTRY(b, cudaMemcpyAsync(d.bpsi + s.bound.off, blob + ps.oBpsi, ps.hb.psi.size() * 4, cudaMemcpyHostToDevice, st));
+  BTRY(b, cudaMemcpyAsync(d.bsample + s.bound.off, blob + ps.oBpos, ps.hb.pos.size() * 4, cudaMemcpyHostToDevice, st));
   BTRY(b, cudaMemcpyAsync(d.bcellStart + s.cells.off, blob + ps.oBcs, ps.hb.cellStart.size() * 4,
                           cudaMemcpyHostToDevice, st));
   BTRY(b, cudaMemsetAsync(d.cellStart + s.cells.off, 0, (size_t)(s.nCells + 2) * 4, st));
@@ -858,8 +858,8 @@ int alloc_arenas(p4a_batch* b) {
        (rc = balloc(b, &d.cellCount, Cc)) ||
        (rc = balloc(b, &d.cellStart, Cc)) || (rc = balloc(b, &d.bcellStart, Cc)) ||
        (rc = balloc(b, &d.scanState, b->scanTilesCap)) || (rc = balloc(b, &d.scanTicket, 4)) ||
-       (rc = balloc(b, &d.errorWord, 4)) || (rc = balloc(b, &d.bpos, b->cfg.max_boundary)) ||
-       (rc = balloc(b, &d.bpsi, b->cfg.max_boundary)) || (rc = balloc(b, &d.bodyAccum, B1 * 4)) ||
+       (rc = balloc(b, &d.errorWord, 4)) || (rc = balloc(b, &d.bsample, b->cfg.max_boundary)) ||
+       (rc = balloc(b, &d.bodyAccum, B1 * 4)) ||
        (rc = balloc(b, &d.bodyCov, B1 * 9)) || (rc = balloc(b, &d.bodyCentre, B1)) ||
        (rc = balloc(b, &d.bodyRef, B1)) || (rc = balloc(b, &d.bodyRot, B1 * 3)) ||
        (rc = balloc(b, &d.bodyInfo, B1)) || (rc = balloc(b, &d.bodyStart, B1)) ||

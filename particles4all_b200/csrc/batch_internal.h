@@ -168,7 +168,7 @@ struct PreparedScene {
   std::vector<int> bodyCounts;
   int nb1 = 1;
   // byte offsets of the pieces in the upload blob
-  size_t oPos = 0, oVel = 0, oPhase = 0, oRest = 0, oBpos = 0, oBpsi = 0, oBcs = 0, oInfo = 0,
+  size_t oPos = 0, oVel = 0, oPhase = 0, oRest = 0, oBpos = 0, oBcs = 0, oInfo = 0,
          oCentre = 0, oRot = 0, oBstart = 0, bytes = 0;
 };
 

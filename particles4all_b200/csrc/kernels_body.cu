@@ -219,7 +219,7 @@ __device__ __forceinline__ void body_match_body(const SimParams& P, const DevSce
       const float4 p0 = __ldg(&d.pos[L][i]);
       const F3 v = {(o.x - p0.x) * P.invDt, (o.y - p0.y) * P.invDt, (o.z - p0.z) * P.invDt};
       d.vel[L ^ 1][i] = make_float4(v.x, v.y, v.z, 0.0f);
-      d.velRho[i] = make_float4(v.x, v.y, v.z, __ldg(&d.density[i]));
+      d.velRho[i] = make_float4(v.x, v.y, v.z, fmaxf(__ldg(&d.density[i]), 0.5f * P.rho0));
     }
   }
 }

@@ -11,9 +11,10 @@
 // With L = P.parity ^ 1 the live copy after the sort, the final positions are in
 // pred[L ^ (iters & 1)]; the velFromPos velocities are in the non-live copy
 // vel[L ^ 1], so the final velocity can be written to vel[L] while neighbours still
-// read the other one. Each pass builds its neighbour list with radius h
-// (neighbours.cuh) and walks it; xsph+normals stores the list for the tension pass,
-// which walks the same positions.
+// read the other one. Each pass walks lambda's last list, or one it builds with radius
+// h (neighbours.cuh); xsph+normals leaves the list for the tension pass, which walks
+// the same positions. The pair terms run two at a time (pair_math.cuh); parameters
+// outside its ranges take the IEEE operations one entry at a time.
 #include <cuda_runtime.h>
 
 #include "neighbours.cuh"
@@ -95,19 +96,35 @@ __device__ __forceinline__ void xsph_finalize_particle(const SimParams& P, const
   const float4 p4 = __ldg(&pred[i]);
   const F3 pi = xyz(p4), vi = xyz(__ldg(&velIn[i]));
   const RowWalk w(P, pi);
-  const uint32_t cap = d.cap;
   const uint32_t count = finish_list(P, d, w, i, pi, pred, cs);
   F3 acc = {0.f, 0.f, 0.f};
-  // g = (velFromPos, density) of neighbour j
-  auto fluid = [&](uint32_t, float4 q, float4 g) {
-    const F3 rij = sub3(pi, xyz(q));
-    const float r2 = dot3(rij, rij);
-    if (r2 >= P.h2) return;  // in the skin of a reused list only
-    const float t = P.h2 - r2;
-    const float f = P.mass * (P.poly6 * t * t * t) / fmaxf(g.w, 0.5f * P.rho0);
-    acc = fma3(f, sub3(xyz(g), vi), acc);
-  };
-  walk_neighbours2<true>(P, w, i, pi, pred, d.velRho, cs, d.nbList, cap, count, fluid);
+  // g = (velFromPos, max(density, rho0 / 2)) of neighbour j
+  if (count != kListOverflow && (P.pairMath & PAIR_XSPH) != 0u) {
+    const F2 h2 = splat2(P.h2), one = splat2(-1.0f), poly = splat2(P.poly6), mass = splat2(-P.mass);
+    walk2g(d.nbList, d.cap, i, count, pred, d.velRho,
+           [&](uint32_t j0, uint32_t j1, float4 q0, float4 q1, float4 g0, float4 g1) {
+      const F3 r0 = sub3(pi, xyz(q0)), r1 = sub3(pi, xyz(q1));
+      const float x0 = dot3(r0, r0), x1 = dot3(r1, r1);
+      const bool in0 = !(x0 >= P.h2) && j0 != i, in1 = !(x1 >= P.h2) && j1 != i;
+      const F2 dens = pack2(g0.w, g1.w);
+      const F2 t = fma2(pack2(x0, x1), one, h2);
+      const F2 f = quot2(mul2(mass, mul2(mul2(mul2(poly, t), t), t)), dens, recip2(dens));
+      float f0, f1;
+      unpack2(f, f0, f1);
+      const F3 v0 = sub3(xyz(g0), vi), v1 = sub3(xyz(g1), vi);
+      if (in0) acc = fma3(f0, v0, acc);
+      if (in1) acc = fma3(f1, v1, acc);
+    });
+  } else {
+    walk_fluid(P, w, i, pi, pred, d.velRho, cs, d.nbList, d.cap, count, [&](float4 q, float4 g) {
+      const F3 rij = sub3(pi, xyz(q));
+      const float r2 = dot3(rij, rij);
+      if (r2 >= P.h2) return;  // in the skin of a reused list only
+      const float t = P.h2 - r2;
+      const float f = P.mass * (P.poly6 * t * t * t) / g.w;
+      acc = fma3(f, sub3(xyz(g), vi), acc);
+    });
+  }
   const F3 corr = mul3(acc, P.xsphC);
   vf = add3(vi, corr);
   d.vel[L][i] = make_float4(vf.x, vf.y, vf.z, 0.0f);
@@ -142,22 +159,52 @@ __device__ __forceinline__ void xsph_normals_body(const SimParams& P, const DevS
   const uint32_t count = finish_list(P, d, w, i, pi, pred, cs);
   d.nbCount[i] = count;
   F3 acc = {0.f, 0.f, 0.f}, nacc = {0.f, 0.f, 0.f};
-  // g = (velFromPos, density) of neighbour j
-  auto fluid = [&](uint32_t, float4 q, float4 g) {
-    const F3 rij = sub3(pi, xyz(q));
-    const float r2 = dot3(rij, rij);
-    if (r2 >= P.h2) return;  // in the skin of a reused list only
-    const float dj = fmaxf(g.w, 0.5f * P.rho0);
-    const float t = P.h2 - r2;  // r2 < h2 here: poly6 without its range test
-    const float f = P.mass * (P.poly6 * t * t * t) / dj;
-    acc = fma3(f, sub3(xyz(g), vi), acc);
-    if (r2 < 1.0e-12f) return;
-    const float rr = sqrtf(r2);
-    const float hr = P.h - rr;
-    const float coef = (P.mass / dj) * (P.spikyGrad * hr * hr / rr);
-    nacc = fma3(coef, rij, nacc);
-  };
-  walk_neighbours2(P, w, i, pi, pred, d.velRho, cs, d.nbList, cap, count, fluid);
+  // g = (velFromPos, max(density, rho0 / 2)) of neighbour j
+  if (count != kListOverflow && (P.pairMath & PAIR_XSPH) != 0u) {
+    const F2 h2 = splat2(P.h2), h = splat2(P.h), one = splat2(-1.0f), poly = splat2(P.poly6);
+    const F2 mass = splat2(-P.mass), cGrad = splat2(-P.spikyGrad);
+    walk2g(d.nbList, cap, i, count, pred, d.velRho,
+           [&](uint32_t j0, uint32_t j1, float4 q0, float4 q1, float4 g0, float4 g1) {
+      const F3 r0 = sub3(pi, xyz(q0)), r1 = sub3(pi, xyz(q1));
+      const float x0 = dot3(r0, r0), x1 = dot3(r1, r1);
+      const bool in0 = !(x0 >= P.h2) && j0 != i, in1 = !(x1 >= P.h2) && j1 != i;
+      const F2 x = pack2(x0, x1);
+      const Root2 root = root2(x);
+      const F2 dens = pack2(g0.w, g1.w), rd = recip2(dens);
+      const F2 t = fma2(x, one, h2);
+      const F2 f = quot2(mul2(mass, mul2(mul2(mul2(poly, t), t), t)), dens, rd);
+      const F2 hr = fma2(root.s, one, h);
+      const F2 grad = quot2(mul2(mul2(cGrad, hr), hr), root.s, root.yn);
+      const F2 coef = mul2(quot2(mass, dens, rd), grad);
+      float f0, f1, k0, k1;
+      unpack2(f, f0, f1);
+      unpack2(coef, k0, k1);
+      const F3 v0 = sub3(xyz(g0), vi), v1 = sub3(xyz(g1), vi);
+      if (in0) {
+        acc = fma3(f0, v0, acc);
+        if (!(x0 < 1.0e-12f)) nacc = fma3(k0, r0, nacc);
+      }
+      if (in1) {
+        acc = fma3(f1, v1, acc);
+        if (!(x1 < 1.0e-12f)) nacc = fma3(k1, r1, nacc);
+      }
+    });
+  } else {
+    walk_fluid(P, w, i, pi, pred, d.velRho, cs, d.nbList, cap, count, [&](float4 q, float4 g) {
+      const F3 rij = sub3(pi, xyz(q));
+      const float r2 = dot3(rij, rij);
+      if (r2 >= P.h2) return;  // in the skin of a reused list only
+      const float dj = g.w;
+      const float t = P.h2 - r2;  // r2 < h2 here: poly6 without its range test
+      const float f = P.mass * (P.poly6 * t * t * t) / dj;
+      acc = fma3(f, sub3(xyz(g), vi), acc);
+      if (r2 < 1.0e-12f) return;
+      const float rr = sqrtf(r2);
+      const float hr = P.h - rr;
+      const float coef = (P.mass / dj) * (P.spikyGrad * hr * hr / rr);
+      nacc = fma3(coef, rij, nacc);
+    });
+  }
   d.corr[i] = make_float4(P.xsphC * acc.x, P.xsphC * acc.y, P.xsphC * acc.z, 0.0f);
   const F3 nrm = {P.h * nacc.x, P.h * nacc.y, P.h * nacc.z};
   d.normal[i] = make_float4(nrm.x, nrm.y, nrm.z, 0.0f);
@@ -183,22 +230,50 @@ __device__ __forceinline__ void tension_finalize_particle(const SimParams& P, co
   const uint32_t count = __ldg(&d.nbCount[i]);  // xsph+normals' list for these positions
   F3 acc = {0.f, 0.f, 0.f};
   // g = (normal, density) of neighbour j
-  auto fluid = [&](uint32_t, float4 q, float4 g) {
-    const F3 rij = sub3(pi, xyz(q));
-    const float r2 = dot3(rij, rij);
-    if (r2 >= P.h2 || r2 < 1.0e-12f) return;
-    const float rr = sqrtf(r2);
-    const float hrr = P.h - rr;
-    const float k = hrr * hrr * hrr * rr * rr * rr;
-    float cw = P.cohes * (2.0f * k - P.cohesTerm);
-    if (2.0f * rr > P.h) cw = P.cohes * k;
-    const float sCoh = -P.tension * P.mass * cw / rr;
-    const F3 fCoh = mul3(rij, sCoh);
-    const F3 fCurv = mul3(sub3(ni, xyz(g)), -P.tension);
-    const float wgt = 2.0f * P.rho0 / (rho + g.w);
-    acc = fma3(wgt, add3(fCoh, fCurv), acc);
-  };
-  walk_neighbours2<true>(P, w, i, pi, pred, d.normRho, cs, d.nbList, cap, count, fluid);
+  if (count != kListOverflow && (P.pairMath & PAIR_TENSION) != 0u) {
+    const F2 h = splat2(P.h), one = splat2(-1.0f), two = splat2(2.0f), cohes = splat2(P.cohes);
+    const F2 term = splat2(-P.cohesTerm), cCoh = splat2(P.tension * P.mass), cRho = splat2(-(2.0f * P.rho0));
+    walk2g(d.nbList, cap, i, count, pred, d.normRho,
+           [&](uint32_t, uint32_t, float4 q0, float4 q1, float4 g0, float4 g1) {
+      const F3 r0 = sub3(pi, xyz(q0)), r1 = sub3(pi, xyz(q1));
+      const float x0 = dot3(r0, r0), x1 = dot3(r1, r1);
+      const bool in0 = !(x0 >= P.h2 || x0 < 1.0e-12f), in1 = !(x1 >= P.h2 || x1 < 1.0e-12f);
+      const Root2 root = root2(pack2(x0, x1));
+      const F2 hr = fma2(root.s, one, h);
+      const F2 k = mul2(mul2(mul2(mul2(mul2(hr, hr), hr), root.s), root.s), root.s);
+      float s0, s1, near0, near1, far0, far1;
+      unpack2(root.s, s0, s1);
+      unpack2(fma2(two, k, term), near0, near1);  // 2 k is exact
+      unpack2(k, far0, far1);
+      const F2 cw = mul2(cohes, pack2(2.0f * s0 > P.h ? far0 : near0, 2.0f * s1 > P.h ? far1 : near1));
+      const F2 sCoh = quot2(mul2(cCoh, cw), root.s, root.yn);
+      const F2 rhoSum = pack2(rho + g0.w, rho + g1.w);
+      const F2 wgt = quot2(cRho, rhoSum, recip2(rhoSum));
+      float c0, c1, w0, w1;
+      unpack2(sCoh, c0, c1);
+      unpack2(wgt, w0, w1);
+      const F3 f0 = add3(mul3(r0, c0), mul3(sub3(ni, xyz(g0)), -P.tension));
+      const F3 f1 = add3(mul3(r1, c1), mul3(sub3(ni, xyz(g1)), -P.tension));
+      if (in0) acc = fma3(w0, f0, acc);
+      if (in1) acc = fma3(w1, f1, acc);
+    });
+  } else {
+    walk_fluid(P, w, i, pi, pred, d.normRho, cs, d.nbList, cap, count, [&](float4 q, float4 g) {
+      const F3 rij = sub3(pi, xyz(q));
+      const float r2 = dot3(rij, rij);
+      if (r2 >= P.h2 || r2 < 1.0e-12f) return;
+      const float rr = sqrtf(r2);
+      const float hrr = P.h - rr;
+      const float k = hrr * hrr * hrr * rr * rr * rr;
+      float cw = P.cohes * (2.0f * k - P.cohesTerm);
+      if (2.0f * rr > P.h) cw = P.cohes * k;
+      const float sCoh = -P.tension * P.mass * cw / rr;
+      const F3 fCoh = mul3(rij, sCoh);
+      const F3 fCurv = mul3(sub3(ni, xyz(g)), -P.tension);
+      const float wgt = 2.0f * P.rho0 / (rho + g.w);
+      acc = fma3(wgt, add3(fCoh, fCurv), acc);
+    });
+  }
   const float4 c0 = d.corr[i];
   const F3 cf = {fmaf(P.dt, acc.x, c0.x), fmaf(P.dt, acc.y, c0.y), fmaf(P.dt, acc.z, c0.z)};
   d.corr[i] = make_float4(cf.x, cf.y, cf.z, 0.0f);
@@ -219,12 +294,17 @@ __device__ __forceinline__ void tension_finalize_body(const SimParams& P, const 
   if (substep == (int)P.subs - 1) block_stats(P, li < P.n, rhoi, vf, d.statsOut + 8 * P.slot);
 }
 
-__global__ void __launch_bounds__(kBlock, 5) k_xsph_finalize(const __grid_constant__ SimParams P,
+// Blocks of 256 per SM, which set the registers a thread may use. 5 (48 registers)
+// spills the pair arithmetic: tension+finalize 469 us on the large scene against 267 us
+// with 4 and 305 us with 3; batched on the 96-scene mix xsph+finalize 350 / 243 / 273 us
+// and tension+finalize 574 / 302 / 284 us with 5 / 4 / 3.
+constexpr int kFinishBlocks = 4, kTensionBlocksBatched = 3;
+__global__ void __launch_bounds__(kBlock, kFinishBlocks) k_xsph_finalize(const __grid_constant__ SimParams P,
                                                              const __grid_constant__ DevScene d,
                                                              int substep) {
   xsph_finalize_body(P, d, blockIdx.x, substep);
 }
-__global__ void __launch_bounds__(kBlock, 5) k_xsph_finalize_b(const __grid_constant__ BatchWork w,
+__global__ void __launch_bounds__(kBlock, kFinishBlocks) k_xsph_finalize_b(const __grid_constant__ BatchWork w,
                                                                const __grid_constant__ DevScene d,
                                                                int substep) {
   for_each_item(w, [&](const SimParams& P, uint32_t t, uint32_t) { xsph_finalize_body(P, d, t, substep); });
@@ -241,18 +321,18 @@ __global__ void __launch_bounds__(TB, MB) k_xsph_normals_b(const __grid_constant
 }
 using PlainFn = void (*)(SimParams, DevScene, int);
 using BatchFn = void (*)(BatchWork, DevScene, int);
-static const PlainFn kNormalsP[kVariants] = {k_xsph_normals<256, 4>, k_xsph_normals<256, 5>,
-                                             k_xsph_normals<256, 3>, k_xsph_normals<128, 8>,
-                                             k_xsph_normals<128, 10>, k_xsph_normals<128, 6>};
-static const BatchFn kNormalsB[kVariants] = {k_xsph_normals_b<256, 4>, k_xsph_normals_b<256, 5>,
-                                             k_xsph_normals_b<256, 3>, k_xsph_normals_b<128, 8>,
-                                             k_xsph_normals_b<128, 10>, k_xsph_normals_b<128, 6>};
-__global__ void __launch_bounds__(kBlock, 5) k_tension_finalize(const __grid_constant__ SimParams P,
+static const PlainFn kNormalsP[kVariants] = {k_xsph_normals<256, 3>, k_xsph_normals<256, 4>,
+                                             k_xsph_normals<256, 2>, k_xsph_normals<128, 6>,
+                                             k_xsph_normals<128, 8>, k_xsph_normals<128, 5>};
+static const BatchFn kNormalsB[kVariants] = {k_xsph_normals_b<256, 3>, k_xsph_normals_b<256, 4>,
+                                             k_xsph_normals_b<256, 2>, k_xsph_normals_b<128, 6>,
+                                             k_xsph_normals_b<128, 8>, k_xsph_normals_b<128, 5>};
+__global__ void __launch_bounds__(kBlock, kFinishBlocks) k_tension_finalize(const __grid_constant__ SimParams P,
                                                                 const __grid_constant__ DevScene d,
                                                                 int substep) {
   tension_finalize_body(P, d, blockIdx.x, substep);
 }
-__global__ void __launch_bounds__(kBlock, 5) k_tension_finalize_b(const __grid_constant__ BatchWork w,
+__global__ void __launch_bounds__(kBlock, kTensionBlocksBatched) k_tension_finalize_b(const __grid_constant__ BatchWork w,
                                                                   const __grid_constant__ DevScene d,
                                                                   int substep) {
   for_each_item(w, [&](const SimParams& P, uint32_t t, uint32_t) { tension_finalize_body(P, d, t, substep); });

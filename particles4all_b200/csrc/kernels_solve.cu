@@ -29,11 +29,58 @@
 
 namespace p4a {
 
-// Called by all 32 lanes of a warp. PF: whether the list walk runs the two-deep
-// prefetch pipeline (measured faster in the batched launches, slower in the plain
-// ones, whose register budget it squeezes; delta's walk always prefetches). (lanes past the scene's end only take part in the
+// One list walk of lambda, two entries at a time; B: the list holds boundary samples
+// (a fluid entry then takes the same path with its own coefficients selected, so that a
+// warp at a wall runs every pair once and not once per kind). The walks are bound by
+// issue slots (77 % of them busy, 80 warp-instructions per entry, a quarter of those in
+// the range tests of an IEEE root and division); with the packed pair arithmetic lambda
+// takes 525 us per launch on the 96-scene mix in halves (728 us one entry at a time with
+// the IEEE operations), delta 327 us (426 us); on the large scene 269 us (289 us) and
+// 178 us (232 us).
+template <bool B>
+__device__ __forceinline__ void lambda_walk(const SimParams& P, const DevScene& d, uint32_t i, uint32_t count, F3 pi,
+                                            const float4* __restrict__ pred, float& rho, F3& gradSum,
+                                            float& sumGrad2) {
+  const F2 one = splat2(-1.0f), h2 = splat2(P.h2), h = splat2(P.h), poly = splat2(P.poly6);
+  const F2 cFluid = splat2(-P.volSpiky);
+  walk2<B>(d.nbList, d.cap, i, count, pred, d.bsample, [&](uint2 e, float4 q0, float4 q1) {
+    const F3 r0 = sub3(pi, xyz(q0)), r1 = sub3(pi, xyz(q1));
+    const float x0 = dot3(r0, r0), x1 = dot3(r1, r1);
+    const bool b0 = B && (e.x & kBoundTag) != 0u, b1 = B && (e.y & kBoundTag) != 0u;
+    const bool in0 = !(x0 >= P.h2 || (b0 && x0 < 1.0e-12f));
+    const bool in1 = !(x1 >= P.h2 || (b1 && x1 < 1.0e-12f)) && e.y != i;
+    const F2 x = pack2(x0, x1);
+    const Root2 root = root2(x);
+    const F2 t = fma2(x, one, h2);
+    const F2 w = mul2(mul2(mul2(poly, t), t), t);
+    const F2 hr = fma2(root.s, one, h);
+    F2 c = cFluid;
+    if constexpr (B)
+      c = pack2(b0 ? -(q0.w * P.invRho0 * P.spikyGrad) : -P.volSpiky, b1 ? -(q1.w * P.invRho0 * P.spikyGrad) : -P.volSpiky);
+    const F2 s = quot2(mul2(mul2(c, hr), hr), root.s, root.yn);
+    float w0, w1, s0, s1;
+    unpack2(w, w0, w1);
+    unpack2(s, s0, s1);
+    auto add = [&](bool in, bool b, float x, float psi, float wk, float sk, F3 r) {
+      const F3 g = mul3(r, sk);
+      const float g2 = dot3(g, g);
+      if (in) {
+        rho = fmaf(b ? psi : P.mass, wk, rho);
+        if (b) {
+          gradSum = fma3(sk, r, gradSum);
+        } else if (x > 1.0e-12f) {
+          gradSum = add3(gradSum, g);
+          sumGrad2 = sumGrad2 + g2;
+        }
+      }
+    };
+    add(in0, b0, x0, q0.w, w0, s0, r0);
+    add(in1, b1, x1, q1.w, w1, s1, r1);
+  });
+}
+
+// Called by all 32 lanes of a warp (lanes past the scene's end only take part in the
 // warp's list builds).
-template <bool PF>
 __device__ __forceinline__ void lambda_body(const SimParams& P, const DevScene& d, uint32_t li, int it) {
   const bool act = li < P.n;
   const uint32_t i = P.pOff + (act ? li : 0u);
@@ -49,7 +96,7 @@ __device__ __forceinline__ void lambda_body(const SimParams& P, const DevScene& 
   if (it == 0 && act) d.nbRef[i] = make_float4(pi.x, pi.y, pi.z, 0.0f);  // the substep's start positions
   uint32_t count = it > 0 && act ? __ldg(&d.nbCount[i]) : kListOverflow;
   const bool need = act && !list_reusable(P, d, it, i, w, cell, count);
-  count = build_lists_warp<true>(P, need, w, i, pi, pred, cs, bcs, d.bpos, d.nbList, cap, P.skinH2, count);
+  count = build_lists_warp<true>(P, need, w, i, pi, pred, cs, bcs, d.bsample, d.nbList, cap, P.skinH2, count);
   if (need) {
     if (count != kListOverflow) count |= (uint32_t)it << kBuildShift;
     d.nbCount[i] = count;
@@ -59,69 +106,49 @@ __device__ __forceinline__ void lambda_body(const SimParams& P, const DevScene& 
   float rho = P.mass * poly6(P, 0.0f);
   F3 gradSum = {0.f, 0.f, 0.f};
   float sumGrad2 = 0.0f;
-  auto fluid = [&](uint32_t, float4 q) {
-    const F3 rij = sub3(pi, xyz(q));
-    const float r2 = dot3(rij, rij);
-    if (r2 >= P.h2) return;  // in the skin of the list only
-    const float t = P.h2 - r2;
-    rho = fmaf(P.mass, P.poly6 * t * t * t, rho);  // poly6 within h
-    if (r2 > 1.0e-12f) {
-      const float rr = sqrtf(r2);
-      const float hr = P.h - rr;
-      const float s = P.volSpiky * hr * hr / rr;
-      const F3 g = mul3(rij, s);
-      gradSum = add3(gradSum, g);
-      sumGrad2 = sumGrad2 + dot3(g, g);
-    }
-  };
-  auto bound = [&](uint32_t k, float4 q) {
-    const F3 rij = sub3(pi, xyz(q));
-    const float r2 = dot3(rij, rij);
-    if (r2 >= P.h2 || r2 < 1.0e-12f) return;
-    const float psi = __ldg(&d.bpsi[k]);
-    const float t = P.h2 - r2;
-    rho = fmaf(psi, P.poly6 * t * t * t, rho);
-    const float rr = sqrtf(r2);
-    const float hr = P.h - rr;
-    const float s = psi * P.invRho0 * P.spikyGrad * hr * hr / rr;
-    gradSum = fma3(s, rij, gradSum);
-  };
-  if (count != kListOverflow) {
-    if constexpr (PF) {
-      walk_list<true>(d.nbList, cap, i, count, pred, d.bpos, [&](uint32_t k, float4 q, bool isB) {
-        if (isB) {
-          bound(k, q);
-        } else {
-          fluid(k, q);
-        }
-      });
+  if (count != kListOverflow && (P.pairMath & PAIR_SOLVE) != 0u) {
+    // warps without a boundary sample in any list skip the kind selects
+    if (__any_sync(__activemask(), (count & kHasBound) != 0u)) {
+      lambda_walk<true>(P, d, i, count, pi, pred, rho, gradSum, sumGrad2);
     } else {
-      // The same terms on one path, fluid or boundary selected per lane: faster
-      // than the branches above in the plain launches (5-9 % per launch where
-      // warps mix wall and interior particles), slower in the pipelined walk of
-      // the batched ones, whose registers it squeezes.
-      walk_list<false, kFetchBound>(d.nbList, cap, i, count, pred, d.bpos, [&](uint32_t k, float4 q, bool isB) {
-        const F3 rij = sub3(pi, xyz(q));
-        const float r2 = dot3(rij, rij);
-        if (r2 >= P.h2 || (isB && r2 < 1.0e-12f)) return;
-        const float psi = isB ? __ldg(&d.bpsi[k]) : 0.0f;
-        const float t = P.h2 - r2;
-        rho = fmaf(isB ? psi : P.mass, P.poly6 * t * t * t, rho);
-        if (isB || r2 > 1.0e-12f) {
-          const float rr = sqrtf(r2);
-          const float hr = P.h - rr;
-          const float c0 = isB ? psi * P.invRho0 * P.spikyGrad : P.volSpiky;
-          const float s = c0 * hr * hr / rr;
-          const F3 g = mul3(rij, s);
-          const F3 gf = add3(gradSum, g), gb = fma3(s, rij, gradSum);
-          gradSum = isB ? gb : gf;
-          const float sg = sumGrad2 + dot3(g, g);
-          sumGrad2 = isB ? sumGrad2 : sg;
-        }
-      });
+      lambda_walk<false>(P, d, i, count, pi, pred, rho, gradSum, sumGrad2);
     }
   } else {
-    walk_direct<true>(P, w, pi, i, pred, cs, bcs, d.bpos, fluid, bound);
+    auto fluid = [&](uint32_t, float4 q) {
+      const F3 rij = sub3(pi, xyz(q));
+      const float r2 = dot3(rij, rij);
+      if (r2 >= P.h2) return;  // in the skin of the list only
+      const float t = P.h2 - r2;
+      rho = fmaf(P.mass, P.poly6 * t * t * t, rho);  // poly6 within h
+      if (r2 > 1.0e-12f) {
+        const float rr = sqrtf(r2);
+        const float hr = P.h - rr;
+        const float s = P.volSpiky * hr * hr / rr;
+        const F3 g = mul3(rij, s);
+        gradSum = add3(gradSum, g);
+        sumGrad2 = sumGrad2 + dot3(g, g);
+      }
+    };
+    auto bound = [&](uint32_t, float4 q) {
+      const F3 rij = sub3(pi, xyz(q));
+      const float r2 = dot3(rij, rij);
+      if (r2 >= P.h2 || r2 < 1.0e-12f) return;
+      const float psi = q.w;
+      const float t = P.h2 - r2;
+      rho = fmaf(psi, P.poly6 * t * t * t, rho);
+      const float rr = sqrtf(r2);
+      const float hr = P.h - rr;
+      const float s = psi * P.invRho0 * P.spikyGrad * hr * hr / rr;
+      gradSum = fma3(s, rij, gradSum);
+    };
+    if (count != kListOverflow) {
+      walk1(d.nbList, cap, i, count, [&](uint32_t e) {
+        if ((e & kBoundTag) != 0u) bound(e, __ldg(&d.bsample[e & ~kBoundTag]));
+        else fluid(e, __ldg(&pred[e]));
+      });
+    } else {
+      walk_direct<true>(P, w, pi, i, pred, cs, bcs, d.bsample, fluid, bound);
+    }
   }
   d.density[i] = rho;
   const float C = rho * P.invRho0 - 1.0f;
@@ -135,57 +162,110 @@ __device__ __forceinline__ void lambda_body(const SimParams& P, const DevScene& 
   d.predLam[i] = make_float4(pi.x, pi.y, pi.z, lam);
 }
 
+// One list walk of delta, two entries at a time (B as in lambda_walk); nc counts the
+// fluid neighbours for sorAverage.
+template <bool B>
+__device__ __forceinline__ void delta_walk(const SimParams& P, const DevScene& d, uint32_t i, uint32_t count,
+                                           float4 self, F3& dsum, F3& dB, float& nc) {
+  const F2 one = splat2(-1.0f), h2 = splat2(P.h2), h = splat2(P.h), poly = splat2(P.poly6);
+  const F2 cGrad = splat2(-P.spikyGrad), wq = splat2(P.sCorrWq), kc = splat2(-P.sCorrK);
+  const F3 pi = xyz(self);
+  walk2<B>(d.nbList, d.cap, i, count, d.predLam, d.bsample, [&](uint2 e, float4 q0, float4 q1) {
+    const F3 r0 = sub3(pi, xyz(q0)), r1 = sub3(pi, xyz(q1));
+    const float x0 = dot3(r0, r0), x1 = dot3(r1, r1);
+    const bool in0 = !(x0 >= P.h2 || x0 < 1.0e-12f), in1 = !(x1 >= P.h2 || x1 < 1.0e-12f);
+    const F2 x = pack2(x0, x1);
+    const Root2 root = root2(x);
+    const F2 hr = fma2(root.s, one, h);
+    const F2 s = quot2(mul2(mul2(cGrad, hr), hr), root.s, root.yn);
+    const F2 t = fma2(x, one, h2);
+    const F2 ratio = mul2(mul2(mul2(mul2(poly, t), t), t), wq);
+    const F2 r2r = mul2(ratio, ratio);
+    const F2 sc = mul2(mul2(kc, r2r), r2r);
+    float c0, c1;
+    unpack2(sc, c0, c1);
+    const float f0 = self.w + q0.w + c0, f1 = self.w + q1.w + c1;
+    if constexpr (B) {
+      const bool b0 = (e.x & kBoundTag) != 0u, b1 = (e.y & kBoundTag) != 0u;
+      float k0, k1;
+      unpack2(mul2(pack2(b0 ? self.w * q0.w : f0, b1 ? self.w * q1.w : f1), s), k0, k1);
+      auto add = [&](bool in, bool b, float coef, F3 r) {
+        if (in && b) dB = fma3(coef, r, dB);
+        if (in && !b) {
+          dsum = fma3(coef, r, dsum);
+          nc += 1.0f;
+        }
+      };
+      add(in0, b0, k0, r0);
+      add(in1, b1, k1, r1);
+    } else {
+      float k0, k1;
+      unpack2(mul2(pack2(f0, f1), s), k0, k1);
+      if (in0) {
+        dsum = fma3(k0, r0, dsum);
+        nc += 1.0f;
+      }
+      if (in1) {
+        dsum = fma3(k1, r1, dsum);
+        nc += 1.0f;
+      }
+    }
+  });
+}
+
 __device__ __forceinline__ void delta_body(const SimParams& P, const DevScene& d, uint32_t li, int it) {
   if (li >= P.n) return;
   const uint32_t i = P.pOff + li;
   const int L = (int)P.parity ^ 1;
   float4* __restrict__ predOut = d.pred[L ^ ((it + 1) & 1)];
-  const uint32_t* __restrict__ cs = d.cellStart + P.cOff;
-  const uint32_t* __restrict__ bcs = d.bcellStart + P.cOff;
   // lambda's (position, lambda) of this iteration: the positions of pred[L ^ (it & 1)]
   const float4* __restrict__ pl = d.predLam;
-  const uint32_t cap = d.cap;
   const float4 self = __ldg(&pl[i]);
   const F3 pi = xyz(self);
-  const float li_ = self.w;
   const uint32_t count = __ldg(&d.nbCount[i]);  // lambda's list for these positions
   F3 dsum = {0.f, 0.f, 0.f}, dB = {0.f, 0.f, 0.f};
   float nc = 1.0f;
-  auto fluid = [&](uint32_t, float4 q) {
-    const F3 rij = sub3(pi, xyz(q));
-    const float r2 = dot3(rij, rij);
-    if (r2 >= P.h2 || r2 < 1.0e-12f) return;
-    const float rr = sqrtf(r2);
-    const float hr = P.h - rr;
-    const float s = P.spikyGrad * hr * hr / rr;
-    const float t = P.h2 - r2;
-    const float ratio = P.poly6 * t * t * t * P.sCorrWq;
-    const float r2r = ratio * ratio;
-    const float sc = -P.sCorrK * r2r * r2r;
-    const float coef = (li_ + q.w + sc) * s;
-    dsum = fma3(coef, rij, dsum);
-    nc += 1.0f;
-  };
-  auto bound = [&](uint32_t k, float4 q) {
-    const F3 rij = sub3(pi, xyz(q));
-    const float r2 = dot3(rij, rij);
-    if (r2 >= P.h2 || r2 < 1.0e-12f) return;
-    const float rr = sqrtf(r2);
-    const float hr = P.h - rr;
-    const float coef = (li_ * __ldg(&d.bpsi[k])) * (P.spikyGrad * hr * hr / rr);
-    dB = fma3(coef, rij, dB);
-  };
-  if (count != kListOverflow) {
-    walk_list<true, kFetchBound>(d.nbList, cap, i, count, pl, d.bpos, [&](uint32_t k, float4 q, bool isB) {
-      if (isB) {
-        bound(k, q);
-      } else {
-        fluid(k, q);
-      }
-    });
+  if (count != kListOverflow && (P.pairMath & PAIR_SOLVE) != 0u) {
+    if (__any_sync(__activemask(), (count & kHasBound) != 0u)) {
+      delta_walk<true>(P, d, i, count, self, dsum, dB, nc);
+    } else {
+      delta_walk<false>(P, d, i, count, self, dsum, dB, nc);
+    }
   } else {
-    const RowWalk w(P, pi);
-    walk_direct<true>(P, w, pi, i, pl, cs, bcs, d.bpos, fluid, bound);
+    const float li_ = self.w;
+    auto fluid = [&](uint32_t, float4 q) {
+      const F3 rij = sub3(pi, xyz(q));
+      const float r2 = dot3(rij, rij);
+      if (r2 >= P.h2 || r2 < 1.0e-12f) return;
+      const float rr = sqrtf(r2);
+      const float hr = P.h - rr;
+      const float s = P.spikyGrad * hr * hr / rr;
+      const float t = P.h2 - r2;
+      const float ratio = P.poly6 * t * t * t * P.sCorrWq;
+      const float r2r = ratio * ratio;
+      const float sc = -P.sCorrK * r2r * r2r;
+      const float coef = (li_ + q.w + sc) * s;
+      dsum = fma3(coef, rij, dsum);
+      nc += 1.0f;
+    };
+    auto bound = [&](uint32_t, float4 q) {
+      const F3 rij = sub3(pi, xyz(q));
+      const float r2 = dot3(rij, rij);
+      if (r2 >= P.h2 || r2 < 1.0e-12f) return;
+      const float rr = sqrtf(r2);
+      const float hr = P.h - rr;
+      const float coef = (li_ * q.w) * (P.spikyGrad * hr * hr / rr);
+      dB = fma3(coef, rij, dB);
+    };
+    if (count != kListOverflow) {
+      walk1(d.nbList, d.cap, i, count, [&](uint32_t e) {
+        if ((e & kBoundTag) != 0u) bound(e, __ldg(&d.bsample[e & ~kBoundTag]));
+        else fluid(e, __ldg(&pl[e]));
+      });
+    } else {
+      const RowWalk w(P, pi);
+      walk_direct<true>(P, w, pi, i, pl, d.cellStart + P.cOff, d.bcellStart + P.cOff, d.bsample, fluid, bound);
+    }
   }
   const F3 dd = {fmaf(dB.x, P.invRho0, dsum.x * P.volume), fmaf(dB.y, P.invRho0, dsum.y * P.volume),
                  fmaf(dB.z, P.invRho0, dsum.z * P.volume)};
@@ -204,7 +284,7 @@ __device__ __forceinline__ void delta_body(const SimParams& P, const DevScene& d
     const float4 p0 = __ldg(&d.pos[L][i]);
     const F3 v = {(o.x - p0.x) * P.invDt, (o.y - p0.y) * P.invDt, (o.z - p0.z) * P.invDt};
     d.vel[L ^ 1][i] = make_float4(v.x, v.y, v.z, 0.0f);
-    d.velRho[i] = make_float4(v.x, v.y, v.z, __ldg(&d.density[i]));
+    d.velRho[i] = make_float4(v.x, v.y, v.z, fmaxf(__ldg(&d.density[i]), 0.5f * P.rho0));
   }
 }
 
@@ -213,12 +293,12 @@ __device__ __forceinline__ void delta_body(const SimParams& P, const DevScene& d
 template <int TB, int MB>
 __global__ void __launch_bounds__(TB, MB) k_lambda(const __grid_constant__ SimParams P,
                                                    const __grid_constant__ DevScene d, int it) {
-  lambda_body<false>(P, d, blockIdx.x * TB + threadIdx.x, it);
+  lambda_body(P, d, blockIdx.x * TB + threadIdx.x, it);
 }
 template <int TB, int MB>
 __global__ void __launch_bounds__(TB, MB) k_lambda_b(const __grid_constant__ BatchWork w,
                                                      const __grid_constant__ DevScene d, int it) {
-  for_each_slice(w, [&](const SimParams& P, uint32_t li) { lambda_body<true>(P, d, li, it); });
+  for_each_slice(w, [&](const SimParams& P, uint32_t li) { lambda_body(P, d, li, it); });
 }
 template <int TB, int MB>
 __global__ void __launch_bounds__(TB, MB) k_delta(const __grid_constant__ SimParams P,
@@ -233,16 +313,13 @@ __global__ void __launch_bounds__(TB, MB) k_delta_b(const __grid_constant__ Batc
 
 using PlainFn = void (*)(SimParams, DevScene, int);
 using BatchFn = void (*)(BatchWork, DevScene, int);
-#define P4A_SHAPES(K, suffix)                                                                        \
-  {K##suffix<256, 4>, K##suffix<256, 5>, K##suffix<256, 6>, K##suffix<128, 8>, K##suffix<128, 10>, \
-   K##suffix<128, 12>}
-#define P4A_SHAPES_D(K, suffix)                                                                      \
-  {K##suffix<256, 5>, K##suffix<256, 4>, K##suffix<256, 6>, K##suffix<128, 10>, K##suffix<128, 8>, \
-   K##suffix<128, 12>}
+#define P4A_SHAPES(K, suffix)                                                                     \
+  {K##suffix<256, 4>, K##suffix<256, 3>, K##suffix<256, 5>, K##suffix<128, 8>, K##suffix<128, 6>, \
+   K##suffix<128, 10>}
 static const PlainFn kLambdaP[kVariants] = P4A_SHAPES(k_lambda, );
 static const BatchFn kLambdaB[kVariants] = P4A_SHAPES(k_lambda, _b);
-static const PlainFn kDeltaP[kVariants] = P4A_SHAPES_D(k_delta, );
-static const BatchFn kDeltaB[kVariants] = P4A_SHAPES_D(k_delta, _b);
+static const PlainFn kDeltaP[kVariants] = P4A_SHAPES(k_delta, );
+static const BatchFn kDeltaB[kVariants] = P4A_SHAPES(k_delta, _b);
 
 static int pick(int kernel, int variant, int64_t n) {
   return variant >= 0 && variant < kVariants ? variant : tuned_variant(kernel, n);

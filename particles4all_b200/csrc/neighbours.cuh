@@ -9,21 +9,23 @@
 //      (h, or h + skin for lists that later Jacobi iterations reuse) to the
 //      particle's neighbour list, in the reference's visiting order: rows z->y,
 //      fluid j ascending, then the row's boundary samples (tagged kBoundTag);
-//   2. walk_list runs the pass's real work over the list, one entry per loop
-//      iteration, every entry re-tested against r^2 < h^2 with the current
-//      positions by the pass itself.
+//   2. walk2 / walk2g run the pass's real work over the list, two entries per loop
+//      iteration (pair_math.cuh), every entry re-tested against r^2 < h^2 with the
+//      current positions by the pass itself, the sums taken in list order.
 // Phase 2 therefore visits exactly the reference's neighbours in exactly its
 // order, so sums are bit-identical, while the expensive in-range work no longer
 // runs warp-wide on every candidate, and the loop has no per-row bookkeeping:
 // lanes of a warp hold different numbers of neighbours per row, so a walk that
 // switches rows inside the loop pays the switch in almost every iteration.
-// The list is stored [entry][particle] (entry k of particle i at k * cap + i), so
-// the lanes of a warp read entry k of 32 consecutive particles with one
-// coalesced load. The particle itself is never listed (it contributes to no
-// pass). A particle with more than kListCap entries is marked kListOverflow and
-// walked with the reference's direct loop instead.
+// The list is stored [entry / 2][particle][2] (list_at), so the lanes of a warp read
+// two entries of 32 consecutive particles with one coalesced 8-byte load. The
+// particle itself is never listed (it contributes to no pass), except that a list of
+// odd length is padded with it: r^2 = 0 contributes to no pass but lambda's density,
+// which tests for it. A particle with more than kListCap entries is marked
+// kListOverflow and walked with the reference's direct loop instead.
 #pragma once
 #include "p4a_math.cuh"
+#include "pair_math.cuh"
 
 namespace p4a {
 
@@ -33,6 +35,11 @@ constexpr uint32_t kBoundTag = 0x80000000u;      // entry = kBoundTag | boundary
 constexpr uint32_t kHasBound = 0x40000000u;      // count flag: the list holds boundary samples
 constexpr uint32_t kCountMask = 0x0000ffffu;
 constexpr int kBuildShift = 16;                  // count bits 16-19: the iteration that built the list
+
+// Place of entry k of particle i in a list array of `cap` particles.
+__device__ __forceinline__ size_t list_at(uint32_t k, uint32_t cap, uint32_t i) {
+  return 2 * ((size_t)(k >> 1) * cap + i) + (k & 1u);
+}
 
 // Row r = 3*(dz+1) + (dy+1), the reference's dz-outer, dy-inner order.
 struct RowWalk {
@@ -63,13 +70,15 @@ __device__ __forceinline__ uint32_t build_list(const SimParams& P, const RowWalk
                                                const uint32_t* __restrict__ bcs,
                                                const float4* __restrict__ bpos, uint32_t* __restrict__ list,
                                                uint32_t cap, float r2lim) {
-  uint32_t c = 0, flags = 0u;
-  uint32_t* __restrict__ out = list + i;  // entry c at list[c * cap + i]
+  uint32_t c = 0, flags = 0u, held = 0u;
+  // entries are stored two at a time: `held` is the first of a pair
+  uint2* __restrict__ out = reinterpret_cast<uint2*>(list) + i;
   auto push = [&](uint32_t e) {
-    if (c < kListCap) {
-      *out = e;
+    if ((c & 1u) != 0u && c < kListCap) {
+      *out = make_uint2(held, e);
       out += cap;
     }
+    held = e;
     c++;
   };
 #pragma unroll 1
@@ -108,6 +117,7 @@ __device__ __forceinline__ uint32_t build_list(const SimParams& P, const RowWalk
       }
     }
   }
+  if ((c & 1u) != 0u && c < kListCap) *out = make_uint2(held, i);
   return c > kListCap ? kListOverflow : c | flags;
 }
 
@@ -139,7 +149,7 @@ __device__ __forceinline__ uint32_t build_list_coop(const SimParams& P, const Ro
       const uint32_t m = __ballot_sync(0xffffffffu, in);
       if (in) {
         const uint32_t pos = c + (uint32_t)__popc(m & below);
-        if (pos < kListCap) list[(size_t)pos * cap + iL] = j;
+        if (pos < kListCap) list[list_at(pos, cap, iL)] = j;
       }
       c += (uint32_t)__popc(m);
     }
@@ -156,7 +166,7 @@ __device__ __forceinline__ uint32_t build_list_coop(const SimParams& P, const Ro
           const uint32_t m = __ballot_sync(0xffffffffu, in);
           if (in) {
             const uint32_t pos = c + (uint32_t)__popc(m & below);
-            if (pos < kListCap) list[(size_t)pos * cap + iL] = kBoundTag | k;
+            if (pos < kListCap) list[list_at(pos, cap, iL)] = kBoundTag | k;
           }
           if (m) flags = kHasBound;
           c += (uint32_t)__popc(m);
@@ -164,6 +174,7 @@ __device__ __forceinline__ uint32_t build_list_coop(const SimParams& P, const Ro
       }
     }
   }
+  if ((c & 1u) != 0u && c < kListCap && lane == 0u) list[list_at(c, cap, iL)] = iL;
   return c > kListCap ? kListOverflow : c | flags;
 }
 
@@ -256,67 +267,55 @@ __device__ __forceinline__ bool list_reusable(const SimParams& P, const DevScene
   return V * 1.00001f <= P.skinHalf;
 }
 
-// Phase 2 over a list of `count` entries: pair(idx, q, isBound) for every entry,
-// with q = fsrc[idx] for a fluid entry and q = bsrc[idx] for a boundary sample
-// (for a pass that skips boundary samples their calls carry an unused q). One callback for both kinds, so that a pass can treat them on one path with
-// per-lane selects where that is cheaper than running both paths in turn for a
-// warp whose lanes hold entries of both kinds. With PF the walk is
-// software pipelined two entries deep: while entry k is processed, the gather of
-// entry k+1 and the list load of entry k+2 are already in flight, so the latency
-// of the dependent list-then-gather chain overlaps the arithmetic of the current
-// pair. The gather address is chosen without a branch, in one of two forms (both
-// give the same q; which is faster depends on the kernel's register budget):
-// kFetchBound for a pass that reads boundary samples from bsrc, and kFetchAny that
-// decides by bsrc != null at run time (a boundary entry of a pass without boundary
-// samples loads the particle's own fsrc[i]).
-enum FetchForm { kFetchAny, kFetchBound };
-template <bool PF = true, FetchForm FORM = kFetchAny, class FPair>
-__device__ __forceinline__ void walk_list(const uint32_t* __restrict__ list, uint32_t cap, uint32_t i,
-                                          uint32_t count, const float4* __restrict__ fsrc,
-                                          const float4* __restrict__ bsrc, FPair&& pair) {
-  count &= kCountMask;
-  if (count == 0u) return;
+// Phase 2: pair(e, q0, q1) for every two entries e.x, e.y of the list (e.y is the
+// particle itself when the count is odd and this is the last pair), with q0, q1 =
+// fsrc[entry] of a fluid entry and, when B, bsrc[sample] of a boundary entry (e still
+// carries its tag). Without B the list holds no boundary samples. The loop is software
+// pipelined: while a pair is processed, the next pair's gathers and the list load after
+// it are in flight, so the latency of the dependent list-then-gather chain overlaps
+// the arithmetic.
+template <bool B, class FPair>
+__device__ __forceinline__ void walk2(const uint32_t* list, uint32_t cap, uint32_t i, uint32_t count,
+                                      const float4* __restrict__ fsrc, const float4* __restrict__ bsrc,
+                                      FPair&& pair) {
+  const uint32_t pairs = ((count & kCountMask) + 1u) >> 1;
+  if (pairs == 0u) return;
   auto fetch = [&](uint32_t e) {
-    const bool b = (e & kBoundTag) != 0u;
-    if constexpr (FORM == kFetchBound) {
-      return __ldg((b ? bsrc : fsrc) + (e & ~kBoundTag));  // a fluid entry has no tag bit
-    } else {
-      const float4* src = b && bsrc ? bsrc : fsrc;
-      const uint32_t idx = b ? (bsrc ? (e & ~kBoundTag) : i) : e;
-      return __ldg(src + idx);
-    }
+    if constexpr (B) return __ldg(((e & kBoundTag) != 0u ? bsrc : fsrc) + (e & ~kBoundTag));
+    return __ldg(fsrc + e);
   };
-  auto visit = [&](uint32_t cur, float4 q) { pair(cur & ~kBoundTag, q, (cur & kBoundTag) != 0u); };
-  const uint32_t* __restrict__ at = list + i;  // entry k of the particle at list[k * cap + i]
-  uint32_t e0 = __ldg(at);
-  if constexpr (PF) {
-    float4 q0 = fetch(e0);
+  // plain loads: the same kernel may have just written the list
+  const uint2* at = reinterpret_cast<const uint2*>(list) + i;
+  uint2 e = *at, en = e;
+  float4 q0 = fetch(e.x), q1 = fetch(e.y);
+  if (pairs > 1u) {
     at += cap;
-    uint32_t e1 = count > 1u ? __ldg(at) : 0u;
-    for (uint32_t k = 1; k <= count; k++) {
-      const uint32_t cur = e0;
-      const float4 qc = q0;
-      if (k < count) {
-        e0 = e1;
-        q0 = fetch(e1);
-        if (k + 1 < count) {
-          at += cap;
-          e1 = __ldg(at);
-        }
-      }
-      visit(cur, qc);
-    }
-  } else {
-    // one entry ahead; the loop runs while a next entry exists, the last entry is
-    // visited after it
-    for (uint32_t k = 1; k < count; k++) {
-      const uint32_t cur = e0;
-      at += cap;
-      e0 = __ldg(at);
-      visit(cur, fetch(cur));
-    }
-    visit(e0, fetch(e0));
+    en = *at;
   }
+  for (uint32_t k = 1u; k <= pairs; k++) {
+    const uint2 ec = e;
+    const float4 c0 = q0, c1 = q1;
+    if (k < pairs) {
+      e = en;
+      q0 = fetch(e.x);
+      q1 = fetch(e.y);
+      if (k + 1u < pairs) {
+        at += cap;
+        en = *at;
+      }
+    }
+    pair(ec, c0, c1);
+  }
+}
+
+// The entries of a list one at a time: visit(entry). For parameters outside the ranges
+// of the pair arithmetic (pair_math_ranges).
+template <class F>
+__device__ __forceinline__ void walk1(const uint32_t* list, uint32_t cap, uint32_t i, uint32_t count,
+                                      F&& visit) {
+  count &= kCountMask;
+#pragma unroll 1
+  for (uint32_t k = 0; k < count; k++) visit(list[list_at(k, cap, i)]);
 }
 
 // The reference's direct loop (particles whose list overflowed): every candidate
@@ -353,79 +352,60 @@ __device__ __forceinline__ void walk_direct(const SimParams& P, const RowWalk& w
   }
 }
 
-// Fluid-only passes (xsph, normals, tension): fluid(j, q, g) for every fluid
-// neighbour entry of the list, q = pred[j] and g = gsrc[j] (the pass's packed
-// per-neighbour values), both loaded in the walk's two-deep pipeline so that
-// neither gather's latency is waited for in the pair's arithmetic; boundary
-// entries of a reused list are skipped. An overflowed list walks the direct loop.
-// PEEL: the loop runs only while a next entry exists and the last two entries are
-// visited after it (no per-entry tests of what is left, the pair term inlined three
-// times), measured faster in the block-form finalize passes and slower elsewhere.
-template <bool PEEL = false, class FFluid>
-__device__ __forceinline__ void walk_neighbours2(const SimParams& P, const RowWalk& w, uint32_t i, F3 pi,
-                                                 const float4* __restrict__ pred,
-                                                 const float4* __restrict__ gsrc,
-                                                 const uint32_t* __restrict__ cs,
-                                                 const uint32_t* __restrict__ list, uint32_t cap, uint32_t count,
-                                                 FFluid&& fluid) {
-  if (count == kListOverflow) {
-    auto none = [](uint32_t, float4) {};
-    walk_direct<false>(P, w, pi, i, pred, cs, nullptr, nullptr,
-                       [&](uint32_t j, float4 q) { fluid(j, q, __ldg(&gsrc[j])); }, none);
-    return;
+// The walk of the fluid-only passes (xsph, normals, tension): pair(j0, j1, q0, q1, g0,
+// g1) for every two entries, q = pred[j] and g = gsrc[j] (the pass's packed
+// per-neighbour values), both gathered in the pipeline. A boundary entry of a reused
+// list is replaced by the particle itself, as the padding is: j == i is skipped by the
+// pass.
+template <class FPair>
+__device__ __forceinline__ void walk2g(const uint32_t* list, uint32_t cap, uint32_t i, uint32_t count,
+                                       const float4* __restrict__ pred, const float4* __restrict__ gsrc,
+                                       FPair&& pair) {
+  const uint32_t pairs = ((count & kCountMask) + 1u) >> 1;
+  if (pairs == 0u) return;
+  auto slot = [&](uint32_t e) { return (e & kBoundTag) != 0u ? i : e; };
+  const uint2* at = reinterpret_cast<const uint2*>(list) + i;
+  uint2 e = *at;
+  uint32_t j0 = slot(e.x), j1 = slot(e.y);
+  float4 q0 = __ldg(pred + j0), q1 = __ldg(pred + j1), g0 = __ldg(gsrc + j0), g1 = __ldg(gsrc + j1);
+  if (pairs > 1u) {
+    at += cap;
+    e = *at;
   }
-  count &= kCountMask;
-  if (count == 0u) return;
-  auto slot = [&](uint32_t e) { return (e & kBoundTag) != 0u ? i : e; };  // a boundary entry loads i
-  const uint32_t* __restrict__ at = list + i;  // entry k of the particle at list[k * cap + i]
-  uint32_t e0 = __ldg(at);
-  float4 q0 = __ldg(pred + slot(e0)), g0 = __ldg(gsrc + slot(e0));
-  if constexpr (PEEL) {
-    uint32_t e1 = 0u;
-    if (count > 1u) {
-      at += cap;
-      e1 = __ldg(at);
-    }
-    auto visit = [&](uint32_t cur, float4 qc, float4 gc) {
-      if ((cur & kBoundTag) == 0u) fluid(cur, qc, gc);
-    };
-    for (uint32_t k = 1; k + 1 < count; k++) {
-      const uint32_t cur = e0;
-      const float4 qc = q0, gc = g0;
-      e0 = e1;
-      q0 = __ldg(pred + slot(e1));
-      g0 = __ldg(gsrc + slot(e1));
-      at += cap;
-      e1 = __ldg(at);
-      visit(cur, qc, gc);
-    }
-    if (count > 1u) {
-      const uint32_t cur = e0;
-      const float4 qc = q0, gc = g0;
-      e0 = e1;
-      q0 = __ldg(pred + slot(e1));
-      g0 = __ldg(gsrc + slot(e1));
-      visit(cur, qc, gc);
-    }
-    visit(e0, q0, g0);
-    return;
-  }
-  at += cap;
-  uint32_t e1 = count > 1u ? __ldg(at) : 0u;
-  for (uint32_t k = 1; k <= count; k++) {
-    const uint32_t cur = e0;
-    const float4 qc = q0, gc = g0;
-    if (k < count) {
-      e0 = e1;
-      q0 = __ldg(pred + slot(e1));
-      g0 = __ldg(gsrc + slot(e1));
-      if (k + 1 < count) {
+  for (uint32_t k = 1u; k <= pairs; k++) {
+    const uint32_t i0 = j0, i1 = j1;
+    const float4 c0 = q0, c1 = q1, h0 = g0, h1 = g1;
+    if (k < pairs) {
+      j0 = slot(e.x);
+      j1 = slot(e.y);
+      q0 = __ldg(pred + j0);
+      q1 = __ldg(pred + j1);
+      g0 = __ldg(gsrc + j0);
+      g1 = __ldg(gsrc + j1);
+      if (k + 1u < pairs) {
         at += cap;
-        e1 = __ldg(at);
+        e = *at;
       }
     }
-    if ((cur & kBoundTag) == 0u) fluid(cur, qc, gc);
+    pair(i0, i1, c0, c1, h0, h1);
   }
+}
+
+// The fluid-only passes one entry at a time: visit(pred[j], gsrc[j]) of every listed
+// fluid entry, or of the reference's direct loop for an overflowed list.
+template <class F>
+__device__ __forceinline__ void walk_fluid(const SimParams& P, const RowWalk& w, uint32_t i, F3 pi,
+                                           const float4* __restrict__ pred, const float4* __restrict__ gsrc,
+                                           const uint32_t* __restrict__ cs, const uint32_t* __restrict__ list,
+                                           uint32_t cap, uint32_t count, F&& visit) {
+  if (count == kListOverflow) {
+    walk_direct<false>(P, w, pi, i, pred, cs, nullptr, nullptr,
+                       [&](uint32_t j, float4 q) { visit(q, __ldg(&gsrc[j])); }, [](uint32_t, float4) {});
+    return;
+  }
+  walk1(list, cap, i, count, [&](uint32_t e) {
+    if ((e & kBoundTag) == 0u) visit(__ldg(&pred[e]), __ldg(&gsrc[e]));
+  });
 }
 
 }  // namespace p4a

@@ -55,7 +55,32 @@ struct SimParams {
   float skinHalf;   // reuse while the displacement bound stays <= this
   float volSpiky;   // volume * spikyGrad rounded to float: the first product of
                     // lambda's fluid gradient term, formed once per substep
+  uint32_t pairMath;  // PAIR_*: passes whose roots and quotients stay in the ranges of
+                      // pair_math.cuh (pair_math_ranges)
 };
+enum : uint32_t { PAIR_SOLVE = 1u, PAIR_XSPH = 2u, PAIR_TENSION = 4u };
+
+// The passes whose pair arithmetic may run without range tests (pair_math.cuh). A root's
+// argument is r^2 in (1e-12, h^2), a quotient's numerator is a constant times a kernel
+// of r. h - r and h^2 - r^2 are zero or at least one unit in the last place (Sterbenz),
+// so a numerator is at least 2^-48 (two factors h - r) or 2^-75 (three factors of
+// h^2 - r^2, or of h - r) of the constants tested here; with these limits every
+// numerator stays above 2^-101 (its remainder is exact) and every quotient is a normal
+// number. Ordinary scenes pass; the others run the IEEE operations one entry at a time.
+inline uint32_t pair_math_ranges(const SimParams& P) {
+  auto in = [](double x, double lo, double hi) { return x >= lo && x <= hi; };
+  const double h = P.h, h2 = h * h, h6 = h2 * h2 * h2;
+  if (!in(h, 0x1p-8, 0x1p8) || !in(P.rho0, 0x1p-40, 0x1p40)) return 0u;
+  uint32_t ok = 0u;
+  const double grad = -(double)P.spikyGrad * h2;
+  if (in(grad, 0x1p-50, 0x1p80) && in(-(double)P.volSpiky * h2, 0x1p-50, 0x1p80)) ok |= PAIR_SOLVE;
+  // density: the particle's own term is its floor, every particle and sample at once its ceiling
+  const double own = (double)P.mass * P.poly6 * h6;
+  const bool density = own >= 0x1p-10 && 2.0 * ((double)P.n * own + ((double)P.nBoundary + 1.0) * P.rho0) <= 0x1p40;
+  if (density && ok && P.mass >= 0x1p-60f) ok |= PAIR_XSPH;
+  if (density && in((double)P.tension * P.mass * P.cohes * h6, 0x1p-20, 0x1p80)) ok |= PAIR_TENSION;
+  return ok;
+}
 
 // Jacobi iterations whose displacement bounds are tracked per substep; later
 // iterations rebuild their masks.
@@ -200,8 +225,9 @@ struct DevScene {
   uint32_t* unordered;
   unsigned long long* scanState;  // epoch-tagged tile states
   uint32_t* scanTicket;
-  float4* bpos;
+  float4* bpos;         // plain scenes only, with bpsi: the buffers p4a_read returns
   float* bpsi;
+  float4* bsample;      // (position, psi) of each boundary sample: one gather in the walks
   uint32_t* bcellStart;
   int32_t* bodyAccum;   // 4 per body
   int32_t* bodyCov;     // 9 per body
@@ -216,7 +242,7 @@ struct DevScene {
   uint32_t* errorWord;
   float4* smoothPos;
   float4* anisoG;
-  uint32_t* nbList;     // [kListCap][cap] neighbour lists (neighbours.cuh), shared by a pair of passes
+  uint32_t* nbList;     // [kListCap / 2][cap][2] neighbour lists (neighbours.cuh), shared by a pair of passes
   uint32_t* nbCount;    // [cap] list length, or kListOverflow
   uint32_t* nbCell;     // [cap] cell index lambda's list was built in
   float* disp;          // [slots][kDispSlots] max |dp| of each iteration of the substep
@@ -225,8 +251,8 @@ struct DevScene {
   uint32_t cellStride;  // cells per cellDisp slot
   float4* nbRef;        // [cap] positions at the start of the substep's iterations
   float4* predLam;      // [cap] (position, lambda) written by lambda for the delta of the same iteration
-  float4* velRho;       // [cap] (velFromPos, density) of the substep's last iteration, the two
-                        // values xsph reads of each neighbour in one gather
+  float4* velRho;       // [cap] (velFromPos, max(density, rho0 / 2)) of the substep's last iteration,
+                        // what xsph reads of each neighbour in one gather
   float4* normRho;      // [cap] (normal, density) written by xsph+normals for tension
   uint32_t cap;         // particle capacity (stride of nbList)
   uint32_t* slotOut;    // optional: sorted position of each input particle

@@ -19,9 +19,9 @@
 namespace p4a {
 
 const LaunchShape kShapes[TK_COUNT][kVariants] = {
-    {{256, 4}, {256, 5}, {256, 6}, {128, 8}, {128, 10}, {128, 12}},   // lambda
-    {{256, 5}, {256, 4}, {256, 6}, {128, 10}, {128, 8}, {128, 12}},   // delta
-    {{256, 4}, {256, 5}, {256, 3}, {128, 8}, {128, 10}, {128, 6}},    // xsph + normals
+    {{256, 4}, {256, 3}, {256, 5}, {128, 8}, {128, 6}, {128, 10}},    // lambda
+    {{256, 4}, {256, 3}, {256, 5}, {128, 8}, {128, 6}, {128, 10}},    // delta
+    {{256, 3}, {256, 4}, {256, 2}, {128, 6}, {128, 8}, {128, 5}},     // xsph + normals
     {{128, 10}, {128, 8}, {128, 12}, {256, 5}, {256, 4}, {64, 20}},   // aniso
 };
 
