@@ -113,6 +113,8 @@ struct p4a_sim {
   // screen-space fluid rendering (p4a_ssfr)
   std::vector<void*> ssfrAllocs;
   SsfrFrame ssfr{};
+  std::vector<void*> ssfrSplats;  // per-splat scratch of the occlusion culling
+  size_t ssfrSplatCap = 0;
   int ssfrW = 0, ssfrH = 0, ssfrMapW = 0, ssfrMapH = 0, ssfrThW = 0, ssfrThH = 0, ssfrGen = 0;
   float4* ssfrBodies = nullptr;
   int ssfrBodyCap = 0;
@@ -694,6 +696,7 @@ int p4a_destroy(p4a_sim* s) {
   if (s->rayImage) cudaFree(s->rayImage);
   if (s->raySurf) cudaFree(s->raySurf);
   if (s->envCube) cudaFree(s->envCube);
+  free_list(s->ssfrSplats);
   if (s->pinned) cudaFreeHost(s->pinned);
   if (s->readEvent) cudaEventDestroy(s->readEvent);
   for (cudaEvent_t e : s->evPool) cudaEventDestroy(e);
@@ -1462,7 +1465,8 @@ int p4a_ssfr(p4a_sim* s, const p4a_ssfr_params* sp, const float* bodies, int32_t
         (rc = dalloc(s, s->ssfrAllocs, &F.eyeZ[0], mapN)) || (rc = dalloc(s, s->ssfrAllocs, &F.eyeZ[1], mapN)) ||
         (rc = dalloc(s, s->ssfrAllocs, &F.raw, mapN)) || (rc = dalloc(s, s->ssfrAllocs, &F.thickMap, thN)) ||
         (rc = dalloc(s, s->ssfrAllocs, &F.thickTmp, thN)) || (rc = dalloc(s, s->ssfrAllocs, &F.bodyT, mapN)) ||
-        (rc = dalloc(s, s->ssfrAllocs, &F.image, (size_t)q.width * q.height)))
+        (rc = dalloc(s, s->ssfrAllocs, &F.image, (size_t)q.width * q.height)) ||
+        (rc = dalloc(s, s->ssfrAllocs, &F.cull.tiles, mapN)) || (rc = dalloc(s, s->ssfrAllocs, &F.cull.listed, 4)))
       return rc;
     s->ssfrMapW = mapW;
     s->ssfrMapH = mapH;
@@ -1484,6 +1488,17 @@ int p4a_ssfr(p4a_sim* s, const p4a_ssfr_params* sp, const float* bodies, int32_t
   F.g = s->anisoG;
   F.phase = s->d.body[s->parity];
   F.bodies = s->ssfrBodies;
+  if ((size_t)std::max(1, s->n) > s->ssfrSplatCap) {
+    CUDA_TRY(s, cudaStreamSynchronize(s->stream));
+    free_list(s->ssfrSplats);
+    s->ssfrSplatCap = 0;
+    const size_t cap = (size_t)std::max(1, s->cap);
+    int rc;
+    if ((rc = dalloc(s, s->ssfrSplats, &F.cull.rect, cap)) || (rc = dalloc(s, s->ssfrSplats, &F.cull.zNear, cap)) ||
+        (rc = dalloc(s, s->ssfrSplats, &F.cull.list, cap)))
+      return rc;
+    s->ssfrSplatCap = cap;
+  }
   // host constants (src/ssfr.js:173-226), in double, stored as float
   const double kPiD = 3.14159265358979323846;
   const double el = q.sun_elevation * kPiD / 180, az = q.sun_azimuth * kPiD / 180;
@@ -1530,6 +1545,9 @@ int p4a_ssfr(p4a_sim* s, const p4a_ssfr_params* sp, const float* bodies, int32_t
     B.size = blurSize;
     const float sigma = std::max((float)blurSize / 3.0f, 1.0e-3f);
     const float twoSigma2 = 2.0f * sigma * sigma;
+  double toScene = 0.0;  // from the eye to the middle of the box
+  for (int k = 0; k < 3; k++) toScene = std::hypot(toScene, q.eye[k] - 0.5 * s->params.box[k]);
+  ssfr_cull_setup(F.cull, q.view, q.proj, q.inv_view_proj, mapW, mapH, q.splat_radius * spacing, toScene);
     for (int i = -blurSize; i <= blurSize; i++) B.w[i + blurSize] = fm_exp(-(float)(i * i) / twoSigma2);
   }
   // depth filter uniforms (src/ssfr.js:151-164, 235-237)

@@ -156,8 +156,27 @@ struct SsfrComp {  // src/ssfr_composite_wgsl.js:2-26
   int32_t width, height, mapW, mapH, thickW, thickH;
   EnvMap env;
 };
+// Occlusion culling of the depth splats (kernels_ssfr.cu): tiles of 2^shift pixels that
+// hold the farthest depth a splat is sure to have drawn over the whole tile.
+struct SsfrCull {
+  uint32_t on;              // the matrices are a rigid view and a perspective (ssfr_cull_setup)
+  int32_t shift, tilesX, tilesY;
+  float p10, p14;           // depth = p14 / distance - p10
+  float transAbs, pvAbs;    // sizes of the view's translation and of proj * view, for the error bounds
+  uint2* rect;              // [count] covered pixels x0 | x1 << 16, y0 | y1 << 16 (0: none)
+  float* zNear;             // [count] no fragment of the splat is nearer
+  uint32_t* list;           // [count] splats left to draw, *listed of them
+  uint32_t* listed;
+  uint32_t* tiles;          // [tilesX * tilesY] float bits
+};
+// Sets on, shift, the tile counts and the constants from the camera (double math);
+// `radius` is the splats' radius and `distance` the scene's distance, which set the tile size.
+void ssfr_cull_setup(SsfrCull& C, const float* view, const float* proj, const float* ivp, int mapW, int mapH,
+                     double radius, double distance);
+
 struct SsfrFrame {
   SsfrSplat depth, thick;
+  SsfrCull cull;
   SsfrBlur blur[2];
   SsfrFilter filter[3];
   int filterSlot[64];
