@@ -97,8 +97,9 @@ struct p4a_sim {
   int anisoGen = 0;
   // surface mesh (p4a_mesh)
   float* meshField[3] = {nullptr, nullptr, nullptr};  // field, normal field, blur scratch
-  uint32_t* meshCounts = nullptr;                     // per voxel, zero between calls
-  uint32_t* meshOffsets = nullptr;                    // [nvox + 1]
+  uint32_t* meshCounts = nullptr;                     // per block of kBlock voxels, zero between calls
+  uint32_t* meshOffsets = nullptr;                    // [blocks + 1]
+  uint2* meshActive = nullptr;                        // [nvox] voxels with triangles (k_mesh_count)
   unsigned long long* meshScan = nullptr;
   uint32_t* meshTicket = nullptr;
   uint2* meshVerts = nullptr;
@@ -108,13 +109,13 @@ struct p4a_sim {
   int32_t meshDim[3] = {0, 0, 0};
   double meshOrigin = 0, meshVoxel = 0;
   int64_t meshTris = 0;
-  size_t meshNvox = 0;  // voxels of the last p4a_mesh: meshOffsets[meshNvox] is its triangle count
+  size_t meshBlocks = 0;  // voxel blocks of the last p4a_mesh: meshOffsets[meshBlocks] is its triangle count
   uint32_t meshEpoch = 0;
   // screen-space fluid rendering (p4a_ssfr)
   std::vector<void*> ssfrAllocs;
-  SsfrFrame ssfr{};
   std::vector<void*> ssfrSplats;  // per-splat scratch of the occlusion culling
   size_t ssfrSplatCap = 0;
+  SsfrFrame ssfr{};
   int ssfrW = 0, ssfrH = 0, ssfrMapW = 0, ssfrMapH = 0, ssfrThW = 0, ssfrThH = 0, ssfrGen = 0;
   float4* ssfrBodies = nullptr;
   int ssfrBodyCap = 0;
@@ -122,6 +123,8 @@ struct p4a_sim {
   int envSize = 0;
   uchar4* rayImage = nullptr;  // p4a_ray
   char* raySurf = nullptr;     // p4a_ray's mesh surface maps, rayCap pixels
+  float2* rayRanges = nullptr; // p4a_ray's ranges of the field, rayRangeCap blocks
+  size_t rayRangeCap = 0;
   size_t rayCap = 0;
   int rayW = 0, rayH = 0;
   bool ready = false;
@@ -688,15 +691,17 @@ int p4a_destroy(p4a_sim* s) {
     if (f) cudaFree(f);
   if (s->meshCounts) cudaFree(s->meshCounts);
   if (s->meshOffsets) cudaFree(s->meshOffsets);
+  if (s->meshActive) cudaFree(s->meshActive);
   if (s->meshScan) cudaFree(s->meshScan);
   if (s->meshTicket) cudaFree(s->meshTicket);
   if (s->meshVerts) cudaFree(s->meshVerts);
   free_list(s->ssfrAllocs);
+  free_list(s->ssfrSplats);
   if (s->ssfrBodies) cudaFree(s->ssfrBodies);
   if (s->rayImage) cudaFree(s->rayImage);
   if (s->raySurf) cudaFree(s->raySurf);
+  if (s->rayRanges) cudaFree(s->rayRanges);
   if (s->envCube) cudaFree(s->envCube);
-  free_list(s->ssfrSplats);
   if (s->pinned) cudaFreeHost(s->pinned);
   if (s->readEvent) cudaEventDestroy(s->readEvent);
   for (cudaEvent_t e : s->evPool) cudaEventDestroy(e);
@@ -1231,6 +1236,7 @@ int p4a_mesh(p4a_sim* s, const p4a_mesh_params* mp, int64_t* triangles) {
     return fail(s, P4A_ERR_CAPACITY, "mesh grid too large");
   const size_t nVerts = (size_t)nv;
   const size_t nvox = (size_t)(dim[0] - 1) * (dim[1] - 1) * (dim[2] - 1);
+  const size_t nBlocks = (size_t)groups((long long)nvox);
   const size_t tris = (size_t)mp->max_triangles;
   after_reads(s, buf_bit(P4A_BUF_MESH_FIELD) | buf_bit(P4A_BUF_MESH_NFIELD) | buf_bit(P4A_BUF_MESH_VERTS));
   if (nVerts > s->meshVertCap || nvox > s->meshVoxCap || tris != s->meshTriCap) {  // src/mesh.js:105-125
@@ -1249,15 +1255,18 @@ int p4a_mesh(p4a_sim* s, const p4a_mesh_params* mp, int64_t* triangles) {
     if (nvox > s->meshVoxCap) {
       if (s->meshCounts) cudaFree(s->meshCounts);
       if (s->meshOffsets) cudaFree(s->meshOffsets);
+      if (s->meshActive) cudaFree(s->meshActive);
       if (s->meshScan) cudaFree(s->meshScan);
       s->meshCounts = s->meshOffsets = nullptr;
+      s->meshActive = nullptr;
       s->meshScan = nullptr;
       s->meshVoxCap = 0;
-      CUDA_TRY(s, cudaMalloc((void**)&s->meshCounts, nvox * 4));
-      CUDA_TRY(s, cudaMemset(s->meshCounts, 0, nvox * 4));
-      CUDA_TRY(s, cudaMalloc((void**)&s->meshOffsets, (nvox + 1) * 4));
-      CUDA_TRY(s, cudaMalloc((void**)&s->meshScan, (size_t)scan_tiles((int)nvox) * 8));
-      CUDA_TRY(s, cudaMemset(s->meshScan, 0, (size_t)scan_tiles((int)nvox) * 8));
+      CUDA_TRY(s, cudaMalloc((void**)&s->meshCounts, nBlocks * 4));
+      CUDA_TRY(s, cudaMemset(s->meshCounts, 0, nBlocks * 4));
+      CUDA_TRY(s, cudaMalloc((void**)&s->meshOffsets, (nBlocks + 1) * 4));
+      CUDA_TRY(s, cudaMalloc((void**)&s->meshActive, nvox * sizeof(uint2)));
+      CUDA_TRY(s, cudaMalloc((void**)&s->meshScan, (size_t)scan_tiles((int)nBlocks) * 8));
+      CUDA_TRY(s, cudaMemset(s->meshScan, 0, (size_t)scan_tiles((int)nBlocks) * 8));
       if (!s->meshTicket) {
         CUDA_TRY(s, cudaMalloc((void**)&s->meshTicket, 16));
         CUDA_TRY(s, cudaMemset(s->meshTicket, 0, 16));
@@ -1295,7 +1304,9 @@ int p4a_mesh(p4a_sim* s, const p4a_mesh_params* mp, int64_t* triangles) {
   const int par = s->parity;
   float* buf[3] = {s->meshField[0], s->meshField[1], s->meshField[2]};
   mark(s, PH_MESH_FIELD);
-  launch_mesh_field(M, s->d.pos[par], s->d.density, s->d.cellStart, s->d.body[par], (uint32_t)s->n, buf[0], st);
+  // predLam is scratch between steps: lambda writes it before delta reads it
+  launch_mesh_field(M, s->d.pos[par], s->d.density, s->d.cellStart, s->d.body[par], (uint32_t)s->n, s->d.predLam,
+                    buf[0], st);
   // blur passes: consecutive passes along one axis run in one launch
   auto blur = [&](int from, int to, int steps) -> int {
     int cur = from;
@@ -1322,19 +1333,20 @@ int p4a_mesh(p4a_sim* s, const p4a_mesh_params* mp, int64_t* triangles) {
     s->nfieldSlot = 0;
   }
   mark(s, PH_MESH_MARCH);
-  launch_mesh_count(M, buf[0], s->meshCounts, (uint32_t)nvox, st);
-  launch_scan(s->meshCounts, s->meshOffsets, (int)nvox, s->meshScan, s->meshTicket, ++s->meshEpoch & 0x3fffffffu,
+  uint32_t* activeCount = s->meshTicket + 1;
+  launch_mesh_count(M, buf[0], s->meshCounts, s->meshActive, activeCount, (uint32_t)nvox, st);
+  launch_scan(s->meshCounts, s->meshOffsets, (int)nBlocks, s->meshScan, s->meshTicket, ++s->meshEpoch & 0x3fffffffu,
               s->d.errorWord, st);
-  launch_mesh_emit(M, buf[0], buf[s->nfieldSlot], s->meshOffsets, (uint32_t)nvox, s->meshVerts, st);
+  launch_mesh_emit(M, buf[0], buf[s->nfieldSlot], s->meshOffsets, s->meshActive, activeCount, s->meshVerts, st);
   mark(s, PH_END);
   CUDA_TRY(s, cudaGetLastError());
   for (int k = 0; k < 3; k++) s->meshDim[k] = dim[k];
   s->meshOrigin = -voxel;
   s->meshVoxel = voxel;
-  s->meshNvox = nvox;
+  s->meshBlocks = nBlocks;
   if (triangles) {
     uint32_t t = 0;
-    CUDA_TRY(s, cudaMemcpyAsync(&t, s->meshOffsets + nvox, 4, cudaMemcpyDeviceToHost, st));
+    CUDA_TRY(s, cudaMemcpyAsync(&t, s->meshOffsets + nBlocks, 4, cudaMemcpyDeviceToHost, st));
     CUDA_TRY(s, cudaStreamSynchronize(st));
     s->meshTris = t;
     *triangles = t;
@@ -1476,6 +1488,17 @@ int p4a_ssfr(p4a_sim* s, const p4a_ssfr_params* sp, const float* bodies, int32_t
     s->ssfrH = q.height;
     s->ssfrGen++;
   }
+  if ((size_t)std::max(1, s->n) > s->ssfrSplatCap) {
+    CUDA_TRY(s, cudaStreamSynchronize(s->stream));
+    free_list(s->ssfrSplats);
+    s->ssfrSplatCap = 0;
+    const size_t cap = (size_t)std::max(1, s->cap);
+    int rc;
+    if ((rc = dalloc(s, s->ssfrSplats, &F.cull.rect, cap)) || (rc = dalloc(s, s->ssfrSplats, &F.cull.zNear, cap)) ||
+        (rc = dalloc(s, s->ssfrSplats, &F.cull.list, cap)))
+      return rc;
+    s->ssfrSplatCap = cap;
+  }
   {
     const int rc = upload_bodies(s, bodies, bodyCount);
     if (rc) return rc;
@@ -1488,17 +1511,6 @@ int p4a_ssfr(p4a_sim* s, const p4a_ssfr_params* sp, const float* bodies, int32_t
   F.g = s->anisoG;
   F.phase = s->d.body[s->parity];
   F.bodies = s->ssfrBodies;
-  if ((size_t)std::max(1, s->n) > s->ssfrSplatCap) {
-    CUDA_TRY(s, cudaStreamSynchronize(s->stream));
-    free_list(s->ssfrSplats);
-    s->ssfrSplatCap = 0;
-    const size_t cap = (size_t)std::max(1, s->cap);
-    int rc;
-    if ((rc = dalloc(s, s->ssfrSplats, &F.cull.rect, cap)) || (rc = dalloc(s, s->ssfrSplats, &F.cull.zNear, cap)) ||
-        (rc = dalloc(s, s->ssfrSplats, &F.cull.list, cap)))
-      return rc;
-    s->ssfrSplatCap = cap;
-  }
   // host constants (src/ssfr.js:173-226), in double, stored as float
   const double kPiD = 3.14159265358979323846;
   const double el = q.sun_elevation * kPiD / 180, az = q.sun_azimuth * kPiD / 180;
@@ -1533,6 +1545,9 @@ int p4a_ssfr(p4a_sim* s, const p4a_ssfr_params* sp, const float* bodies, int32_t
   };
   splat(F.depth, mapW, mapH, 0.0, (double)q.depth_cull_neighbours);
   splat(F.thick, tw, th, thickRadius, 0.0);
+  double toScene = 0.0;  // from the eye to the middle of the box
+  for (int k = 0; k < 3; k++) toScene = std::hypot(toScene, q.eye[k] - 0.5 * s->params.box[k]);
+  ssfr_cull_setup(F.cull, q.view, q.proj, q.inv_view_proj, mapW, mapH, q.splat_radius * spacing, toScene);
   // thickness blur (src/ssfr.js:227-233)
   const int blurSize = q.thickness_filter_size == 0 ? 0
                        : (tw < mapW ? std::max(1, q.thickness_filter_size >> 1) : q.thickness_filter_size);
@@ -1545,9 +1560,6 @@ int p4a_ssfr(p4a_sim* s, const p4a_ssfr_params* sp, const float* bodies, int32_t
     B.size = blurSize;
     const float sigma = std::max((float)blurSize / 3.0f, 1.0e-3f);
     const float twoSigma2 = 2.0f * sigma * sigma;
-  double toScene = 0.0;  // from the eye to the middle of the box
-  for (int k = 0; k < 3; k++) toScene = std::hypot(toScene, q.eye[k] - 0.5 * s->params.box[k]);
-  ssfr_cull_setup(F.cull, q.view, q.proj, q.inv_view_proj, mapW, mapH, q.splat_radius * spacing, toScene);
     for (int i = -blurSize; i <= blurSize; i++) B.w[i + blurSize] = fm_exp(-(float)(i * i) / twoSigma2);
   }
   // depth filter uniforms (src/ssfr.js:151-164, 235-237)
@@ -1727,10 +1739,20 @@ int p4a_ray(p4a_sim* s, const p4a_ray_params* rp, const float* bodies, int32_t b
     CUDA_TRY(s, cudaMalloc((void**)&s->raySurf, px * (8 + 4 + 16)));
     s->rayCap = px;
   }
+  RayParams R{};
+  ray_range_dims(s->meshDim, R.rangeDim);
+  const size_t blocks = (size_t)R.rangeDim[0] * R.rangeDim[1] * R.rangeDim[2];
+  if (blocks > s->rayRangeCap) {
+    CUDA_TRY(s, cudaStreamSynchronize(s->stream));
+    if (s->rayRanges) cudaFree(s->rayRanges);
+    s->rayRanges = nullptr;
+    s->rayRangeCap = 0;
+    CUDA_TRY(s, cudaMalloc((void**)&s->rayRanges, blocks * sizeof(float2)));
+    s->rayRangeCap = blocks;
+  }
   int rc = upload_bodies(s, bodies, bodyCount);
   if (rc) return rc;
   const p4a_ray_params& q = *rp;
-  RayParams R{};
   memcpy(R.ivp, q.inv_view_proj, 64);
   memcpy(R.iv, q.inv_view, 64);
   memcpy(R.view, q.view, 64);
@@ -1778,9 +1800,9 @@ int p4a_ray(p4a_sim* s, const p4a_ray_params* rp, const float* bodies, int32_t b
   unsigned long long* key = (unsigned long long*)(s->raySurf + px * 16);
   float* surfZ = (float*)(s->raySurf + px * 24);
   if (R.useSurface)
-    launch_surface(R, s->meshVerts, s->meshOffsets + s->meshNvox, (uint32_t)s->meshTriCap, R.gridOrigin, R.vertDim,
+    launch_surface(R, s->meshVerts, s->meshOffsets + s->meshBlocks, (uint32_t)s->meshTriCap, R.gridOrigin, R.vertDim,
                    R.voxel, key, surfZ, surfN, s->stream);
-  launch_ray(R, s->meshField[s->fieldSlot], s->ssfrBodies, surfZ, surfN, s->rayImage, s->stream);
+  launch_ray(R, s->meshField[s->fieldSlot], s->rayRanges, s->ssfrBodies, surfZ, surfN, s->rayImage, s->stream);
   mark(s, PH_END);
   CUDA_TRY(s, cudaGetLastError());
   s->rayW = q.width;

@@ -34,22 +34,26 @@ struct Cell {
   float d000, d100, d010, d110, d001, d101, d011, d111;
 };
 
-__device__ __forceinline__ float fget(const RayParams& R, const float* __restrict__ field, int x, int y, int z) {
-  x = min(max(x, 0), R.vertDim[0] - 1);
-  y = min(max(y, 0), R.vertDim[1] - 1);
-  z = min(max(z, 0), R.vertDim[2] - 1);
-  return __ldg(&field[((size_t)z * R.vertDim[1] + y) * R.vertDim[0] + x]);
-}
+// The eight corners of a cell, coordinates clamped to the grid (at most 2^31 vertices:
+// 32-bit indices).
 __device__ __forceinline__ Cell cell_at(const RayParams& R, const float* __restrict__ field, int cx, int cy, int cz) {
+  const uint32_t nx = (uint32_t)R.vertDim[0], ny = (uint32_t)R.vertDim[1];
+  const uint32_t x0 = (uint32_t)min(max(cx, 0), R.vertDim[0] - 1), x1 = (uint32_t)min(max(cx + 1, 0), R.vertDim[0] - 1);
+  const uint32_t y0 = (uint32_t)min(max(cy, 0), R.vertDim[1] - 1), y1 = (uint32_t)min(max(cy + 1, 0), R.vertDim[1] - 1);
+  const uint32_t z0 = (uint32_t)min(max(cz, 0), R.vertDim[2] - 1) * ny, z1 = (uint32_t)min(max(cz + 1, 0), R.vertDim[2] - 1) * ny;
+  const float* __restrict__ r00 = field + (z0 + y0) * nx;
+  const float* __restrict__ r10 = field + (z0 + y1) * nx;
+  const float* __restrict__ r01 = field + (z1 + y0) * nx;
+  const float* __restrict__ r11 = field + (z1 + y1) * nx;
   Cell k;
-  k.d000 = fget(R, field, cx, cy, cz);
-  k.d100 = fget(R, field, cx + 1, cy, cz);
-  k.d010 = fget(R, field, cx, cy + 1, cz);
-  k.d110 = fget(R, field, cx + 1, cy + 1, cz);
-  k.d001 = fget(R, field, cx, cy, cz + 1);
-  k.d101 = fget(R, field, cx + 1, cy, cz + 1);
-  k.d011 = fget(R, field, cx, cy + 1, cz + 1);
-  k.d111 = fget(R, field, cx + 1, cy + 1, cz + 1);
+  k.d000 = __ldg(r00 + x0);
+  k.d100 = __ldg(r00 + x1);
+  k.d010 = __ldg(r10 + x0);
+  k.d110 = __ldg(r10 + x1);
+  k.d001 = __ldg(r01 + x0);
+  k.d101 = __ldg(r01 + x1);
+  k.d011 = __ldg(r11 + x0);
+  k.d111 = __ldg(r11 + x1);
   return k;
 }
 __device__ __forceinline__ float tri_local(const Cell& k, F3 u) {
@@ -169,12 +173,53 @@ __device__ __forceinline__ float body_scene_dist(const RayParams& R, const float
 }
 __device__ __forceinline__ float signf(float x) { return x > 0.0f ? 1.0f : (x < 0.0f ? -1.0f : 0.0f); }
 
+// The field's range over blocks of kRangeCells^3 cells, each grown by one cell on every
+// side (minimum, maximum; the whole line when a value is NaN): where a block is all air
+// or all fluid, the march has no crossing to look for and the optical depth no field to
+// interpolate. At 1080p on the 250,000-particle scene marching the field took 1,106 us
+// without them and 573 us with them, the pass on the mesh surface 240 and 221 us
+// (quotients and ranges together).
+constexpr int kRangeShift = 2, kRangeCells = 1 << kRangeShift;
+__device__ __forceinline__ float2 range_at(const RayParams& R, const float2* __restrict__ ranges, int cx, int cy,
+                                           int cz) {
+  const int bx = min(max(cx >> kRangeShift, 0), R.rangeDim[0] - 1), by = min(max(cy >> kRangeShift, 0), R.rangeDim[1] - 1);
+  const int bz = min(max(cz >> kRangeShift, 0), R.rangeDim[2] - 1);
+  return __ldg(&ranges[(uint32_t)((bz * R.rangeDim[1] + by) * R.rangeDim[0] + bx)]);
+}
+// One warp per block.
+__global__ void __launch_bounds__(128) k_ray_ranges(const __grid_constant__ RayParams R,
+                                                    const float* __restrict__ field, float2* __restrict__ ranges) {
+  const int b = (int)(blockIdx.x * 4 + (threadIdx.x >> 5)), lane = (int)threadIdx.x & 31;
+  if (b >= R.rangeDim[0] * R.rangeDim[1] * R.rangeDim[2]) return;  // whole warps
+  const int bx = b % R.rangeDim[0], by = b / R.rangeDim[0] % R.rangeDim[1], bz = b / (R.rangeDim[0] * R.rangeDim[1]);
+  constexpr int kSide = kRangeCells + 3;  // vertices per axis; a lane takes rows along x
+  float lo = INFINITY, hi = -INFINITY;
+  for (int row = lane; row < kSide * kSide; row += 32) {
+    const int y = min(max(by * kRangeCells - 1 + row % kSide, 0), R.vertDim[1] - 1);
+    const int z = min(max(bz * kRangeCells - 1 + row / kSide, 0), R.vertDim[2] - 1);
+    const float* __restrict__ f = field + (uint32_t)((z * R.vertDim[1] + y) * R.vertDim[0]);
+#pragma unroll
+    for (int k = 0; k < kSide; k++) {
+      const float v = __ldg(f + min(max(bx * kRangeCells - 1 + k, 0), R.vertDim[0] - 1));
+      lo = v != v ? -INFINITY : fminf(lo, v);
+      hi = v != v ? INFINITY : fmaxf(hi, v);
+    }
+  }
+#pragma unroll
+  for (int o = 16; o > 0; o >>= 1) {
+    lo = fminf(lo, __shfl_xor_sync(0xffffffffu, lo, o));
+    hi = fmaxf(hi, __shfl_xor_sync(0xffffffffu, hi, o));
+  }
+  if (lane == 0) ranges[b] = make_float2(lo, hi);
+}
+
 struct March {
   float t;
   F3 pos, nrm;
 };
 __device__ __forceinline__ March march(const RayParams& R, const float* __restrict__ field,
-                                       const float4* __restrict__ bdata, F3 ro, F3 rd, float tStart, float tEnd) {
+                                       const float2* __restrict__ ranges, const float4* __restrict__ bdata, F3 ro,
+                                       F3 rd, float tStart, float tEnd) {
   March out;
   out.t = -1.0f;
   out.pos = {0.f, 0.f, 0.f};
@@ -200,10 +245,15 @@ __device__ __forceinline__ March march(const RayParams& R, const float* __restri
     }
   }
   float t = tStart;
+  // A segment is interpolated by the cubic through four of its points, which is the
+  // field along it up to rounding: in a block whose range stays 1 % off the iso level no
+  // piece of it can bracket that level.
+  const float below = R.iso * 0.99f, above = R.iso * 1.01f;
   for (int i = 0; i < 4096; i++) {
     const float tNext = fminf(fminf(tMax[0], tMax[1]), tMax[2]);
     const float segEnd = fminf(tNext, tEnd);
-    if (segEnd > t) {
+    const float2 range = range_at(R, ranges, c[0], c[1], c[2]);
+    if (segEnd > t && !(R.iso > 0.0f && range.x >= 0.0f && (range.y <= below || range.x >= above))) {
       const Cell k = cell_at(R, field, c[0], c[1], c[2]);
       const F3 u0 = {g0.x + gd.x * t - (float)c[0], g0.y + gd.y * t - (float)c[1], g0.z + gd.z * t - (float)c[2]};
       const float span = segEnd - t;
@@ -241,8 +291,8 @@ __device__ __forceinline__ March march(const RayParams& R, const float* __restri
   }
   return out;
 }
-__device__ __forceinline__ float optical_depth(const RayParams& R, const float* __restrict__ field, F3 ro, F3 rd,
-                                               float tMax) {
+__device__ __forceinline__ float optical_depth(const RayParams& R, const float* __restrict__ field,
+                                               const float2* __restrict__ ranges, F3 ro, F3 rd, float tMax) {
   const F3 lo = f3(R.gridOrigin);
   const F3 hi = {lo.x + R.voxel * (float)(R.vertDim[0] - 1), lo.y + R.voxel * (float)(R.vertDim[1] - 1),
                  lo.z + R.voxel * (float)(R.vertDim[2] - 1)};
@@ -252,12 +302,46 @@ __device__ __forceinline__ float optical_depth(const RayParams& R, const float* 
   const float b = fminf(fmaxf(s.t1, 0.0f), tMax);
   if (b <= a) return 0.0f;
   const float dt = (b - a) / (float)R.thickSteps;
+  const float e0 = R.iso * 0.55f, range = R.iso * 1.45f - e0;
+  // The sample's grid coordinates and its place in the iso band are quotients by the
+  // same two numbers in every step: with their reciprocals rounded once (pair_math.cuh),
+  // each is the IEEE quotient in three operations instead of ten. Numerators are zero or
+  // far above the underflow limit (differences of values of the scene's size).
+  auto quot = [](float num, float den, float yn) {
+    const float qn = num * yn;
+    return -fmaf(fmaf(den, qn, num), yn, qn);
+  };
+  const bool fast = R.voxel > 1.0e-9f && R.voxel < 1.0e9f && range > 1.0e-9f && range < 1.0e9f;
   float acc = 0.0f;
-  for (int i = 0; i < R.thickSteps; i++) {
-    const float t = a + ((float)i + 0.5f) * dt;
-    const F3 q = {(ro.x + rd.x * t - lo.x) / R.voxel, (ro.y + rd.y * t - lo.y) / R.voxel,
-                  (ro.z + rd.z * t - lo.z) / R.voxel};
-    acc += smooth(R.iso * 0.55f, R.iso * 1.45f, tri_at(R, field, q));
+  if (fast) {
+    const float yv = -1.0f / R.voxel, yr = -1.0f / range;
+    // Most samples lie deep in the air or in the fluid: their cell, to within the one
+    // cell by which the ranges are grown, is in a block below or above the whole band
+    // (by more than three lerps can round), where the smoothstep is exactly 0 or 1.
+    const float air = e0 * 0.9999f, water = R.iso * 1.45f * 1.0001f;
+    const F3 g0 = {-yv * (ro.x - lo.x), -yv * (ro.y - lo.y), -yv * (ro.z - lo.z)};
+    const F3 gd = {-yv * rd.x, -yv * rd.y, -yv * rd.z};
+    for (int i = 0; i < R.thickSteps; i++) {
+      const float t = a + ((float)i + 0.5f) * dt;
+      const float2 band = range_at(R, ranges, (int)floorf(fmaf(gd.x, t, g0.x)), (int)floorf(fmaf(gd.y, t, g0.y)),
+                                   (int)floorf(fmaf(gd.z, t, g0.z)));
+      if (band.y <= air) continue;
+      if (band.x >= water) {
+        acc += 1.0f;
+        continue;
+      }
+      const F3 q = {quot(ro.x + rd.x * t - lo.x, R.voxel, yv), quot(ro.y + rd.y * t - lo.y, R.voxel, yv),
+                    quot(ro.z + rd.z * t - lo.z, R.voxel, yv)};
+      const float s = clampf(quot(tri_at(R, field, q) - e0, range, yr), 0.0f, 1.0f);
+      acc += s * s * (3.0f - 2.0f * s);
+    }
+  } else {
+    for (int i = 0; i < R.thickSteps; i++) {
+      const float t = a + ((float)i + 0.5f) * dt;
+      const F3 q = {(ro.x + rd.x * t - lo.x) / R.voxel, (ro.y + rd.y * t - lo.y) / R.voxel,
+                    (ro.z + rd.z * t - lo.z) / R.voxel};
+      acc += smooth(e0, R.iso * 1.45f, tri_at(R, field, q));
+    }
   }
   return acc * dt;
 }
@@ -433,9 +517,10 @@ __global__ void k_surf_resolve(const __grid_constant__ RayParams R, const __grid
   surfN[o] = nn;
 }
 
-__global__ void k_ray(const __grid_constant__ RayParams R, const float* __restrict__ field,
-                      const float4* __restrict__ bdata, const float* __restrict__ surfZ,
-                      const float4* __restrict__ surfN, uchar4* __restrict__ image) {
+__global__ void __launch_bounds__(128, 8) k_ray(const __grid_constant__ RayParams R, const float* __restrict__ field,
+                      const float2* __restrict__ ranges, const float4* __restrict__ bdata,
+                      const float* __restrict__ surfZ, const float4* __restrict__ surfN,
+                      uchar4* __restrict__ image) {
   const int x = blockIdx.x * blockDim.x + threadIdx.x, y = blockIdx.y;
   if (x >= R.width || y >= R.height) return;
   const float nx = ((float)x + 0.5f) / (float)R.width * 2.0f - 1.0f;
@@ -469,7 +554,7 @@ __global__ void k_ray(const __grid_constant__ RayParams R, const float* __restri
   } else {
     const Slab slab = box_hit(ro, rd, volLo, volHi);
     if (slab.hit) {
-      const March m = march(R, field, bdata, ro, rd, fmaxf(slab.t0, 0.0f) + 1.0e-5f, slab.t1);
+      const March m = march(R, field, ranges, bdata, ro, rd, fmaxf(slab.t0, 0.0f) + 1.0e-5f, slab.t1);
       tHit = m.t;
       hit = m.pos;
     }
@@ -510,7 +595,7 @@ __global__ void k_ray(const __grid_constant__ RayParams R, const float* __restri
       trans = background(R, ro2, refrDir);
     }
     const float tSolid = st.t >= 0.0f ? st.t : 1.0e30f;
-    thick = optical_depth(R, field, ro2, refrDir, tSolid);
+    thick = optical_depth(R, field, ranges, ro2, refrDir, tSolid);
     trans = {trans.x * fm_exp(-R.absorb[0] * thick), trans.y * fm_exp(-R.absorb[1] * thick),
              trans.z * fm_exp(-R.absorb[2] * thick)};
     col = lerp3(trans, refl, kS);
@@ -569,12 +654,17 @@ void launch_surface(const RayParams& R, const uint2* verts, const uint32_t* tota
   k_surf_resolve<<<rgrid, tpb, 0, st>>>(R, G, verts, key, surfZ, surfN);
 }
 
-void launch_ray(const RayParams& R, const float* field, const float4* bodies, const float* surfZ,
+void ray_range_dims(const int32_t vertDim[3], int32_t dim[3]) {
+  for (int a = 0; a < 3; a++) dim[a] = (vertDim[a] - 2) / kRangeCells + 1;
+}
+
+void launch_ray(const RayParams& R, const float* field, float2* ranges, const float4* bodies, const float* surfZ,
                 const float4* surfN, uchar4* image, cudaStream_t st) {
   const int tpb = 128;
   const dim3 grid((R.width + tpb - 1) / tpb, R.height);
-  count_launches(1);
-  k_ray<<<grid, tpb, 0, st>>>(R, field, bodies, surfZ, surfN, image);
+  count_launches(2);
+  k_ray_ranges<<<(R.rangeDim[0] * R.rangeDim[1] * R.rangeDim[2] + 3) / 4, tpb, 0, st>>>(R, field, ranges);
+  k_ray<<<grid, tpb, 0, st>>>(R, field, ranges, bodies, surfZ, surfN, image);
 }
 
 }  // namespace p4a

@@ -210,6 +210,7 @@ struct RayParams {
   float cosDeg[4];
   int32_t useSurface;
   float view[16], vp[16];  // view, proj * view (mesh surface pass)
+  int32_t rangeDim[3];     // blocks of the field's ranges (kernels_ray.cu)
   EnvMap env;
 };
 // The mesh surface pass (src/mesh.js:380-396, src/mesh_wgsl.js:240-321 vs + fsSurf):
@@ -218,7 +219,9 @@ struct RayParams {
 void launch_surface(const RayParams& R, const uint2* verts, const uint32_t* total, uint32_t cap,
                     const float gridOrigin[3], const int32_t vertDim[3], float voxel,
                     unsigned long long* key, float* surfZ, float4* surfN, cudaStream_t st);
-void launch_ray(const RayParams& R, const float* field, const float4* bodies, const float* surfZ,
+// `ranges`: scratch, one entry per block of ray_range_dims(vertDim).
+void ray_range_dims(const int32_t vertDim[3], int32_t dim[3]);
+void launch_ray(const RayParams& R, const float* field, float2* ranges, const float4* bodies, const float* surfZ,
                 const float4* surfN, uchar4* image, cudaStream_t st);
 
 // Device error word bits (set by kernels, read by the host at sync points).
@@ -418,11 +421,13 @@ void launch_hose_emit(const HoseEmit& H, const DevScene& d, int parity, int pred
 
 // ---- surface mesh (kernels_mesh.cu) ----
 void launch_mesh_field(const MeshParams& M, const float4* pos, const float* rho, const uint32_t* cs,
-                       const uint4* body, uint32_t n, float* field, cudaStream_t st);
+                       const uint4* body, uint32_t n, float4* weights, float* field, cudaStream_t st);
 cudaError_t launch_mesh_blur(const MeshParams& M, const float* src, float* dst, int axis, int passes,
                              cudaStream_t st);
-void launch_mesh_count(const MeshParams& M, const float* field, uint32_t* counts, uint32_t nvox, cudaStream_t st);
-void launch_mesh_emit(const MeshParams& M, const float* field, const float* nfield, const uint32_t* offsets,
-                      uint32_t nvox, uint2* verts, cudaStream_t st);
+// blockSum: triangles of each block of kBlock voxels; active: voxels with triangles, *activeCount of them.
+void launch_mesh_count(const MeshParams& M, const float* field, uint32_t* blockSum, uint2* active,
+                       uint32_t* activeCount, uint32_t nvox, cudaStream_t st);
+void launch_mesh_emit(const MeshParams& M, const float* field, const float* nfield, const uint32_t* blockOffset,
+                      const uint2* active, const uint32_t* activeCount, uint2* verts, cudaStream_t st);
 
 }  // namespace p4a

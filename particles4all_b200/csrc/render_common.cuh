@@ -197,7 +197,8 @@ __device__ __forceinline__ F3 sky_color(const U& C, F3 d) {
   F3 c = lerp3(haze, mid, smooth(0.0f, 0.16f, h));
   c = lerp3(c, zenith, smooth(0.10f, 0.85f, h));
   const float s = fmaxf(dot3(d, f3(C.sunDir)), 0.0f);
-  const float p1 = fm_pow(s, 3000.0f), p2 = fm_pow(s, 24.0f);
+  // exp underflows to 0 below -104, which 3000 log(0.96) = -122 is well past
+  const float p1 = s < 0.96f ? 0.0f : fm_pow(s, 3000.0f), p2 = fm_pow(s, 24.0f);
   c = {c.x + 1.00f * p1 * 14.0f, c.y + 0.96f * p1 * 14.0f, c.z + 0.88f * p1 * 14.0f};
   c = {c.x + 1.00f * p2 * 0.20f, c.y + 0.92f * p2 * 0.20f, c.z + 0.78f * p2 * 0.20f};
   return c;
