@@ -23,25 +23,37 @@
 
 namespace p4a {
 
-__device__ __forceinline__ void key_count_body(const SimParams& P, const DevScene& d, uint32_t li) {
-  if (d.bodyFill && li < P.nBodies) d.bodyFill[P.bOff + li] = 0u;
+// One thread takes N particles `step` apart, so that the loads and the atomics of all of
+// them are in flight together: the pass is bound by the latency of the atomic whose
+// returned base each warp waits for.
+template <int N>
+__device__ __forceinline__ void key_count_body(const SimParams& P, const DevScene& d, uint32_t li, uint32_t step) {
+  if (d.bodyFill)
+    for (int q = 0; q < N; q++)
+      if (li + q * step < P.nBodies) d.bodyFill[P.bOff + li + q * step] = 0u;
   if (d.disp && li < (uint32_t)kDispSlots) d.disp[P.slot * kDispSlots + li] = 0.0f;
-  const bool act = li < P.n;
-  const uint32_t i = P.pOff + li;
-  uint32_t k = 0xffffffffu;
-  if (act) {
-    F3 v, pr;
-    predict_one(P, __ldg(&d.pos[P.parity][i]), __ldg(&d.vel[P.parity][i]), v, pr);
-    k = P.cOff + cell_index(P, cell_of(P, pr));
+  const int lane = threadIdx.x & 31;
+  uint32_t k[N], base[N];
+  unsigned peers[N];
+  float4 p4[N], v4[N];
+#pragma unroll
+  for (int q = 0; q < N; q++) {
+    const uint32_t i = P.pOff + li + q * step;
+    p4[q] = v4[q] = make_float4(0.0f, 0.0f, 0.0f, 0.0f);
+    if (li + q * step < P.n) {
+      p4[q] = __ldg(&d.pos[P.parity][i]);
+      v4[q] = __ldg(&d.vel[P.parity][i]);
+    }
   }
-  const unsigned peers = __match_any_sync(0xffffffffu, k);
-  if (act) {
-    const int lane = threadIdx.x & 31;
-    const int leader = __ffs(peers) - 1;
-    const uint32_t lt = peers & ((1u << lane) - 1u);
-    uint32_t base = 0;
-    if (lane == leader) {
-      base = atomicAdd(&d.cellCount[k], (uint32_t)__popc(peers));
+#pragma unroll
+  for (int q = 0; q < N; q++) {
+    F3 v, pr;
+    predict_one(P, p4[q], v4[q], v, pr);
+    k[q] = li + q * step < P.n ? P.cOff + cell_index(P, cell_of(P, pr)) : 0xffffffffu;
+    peers[q] = __match_any_sync(0xffffffffu, k[q]);
+    base[q] = 0u;
+    if (k[q] != 0xffffffffu && lane == __ffs(peers[q]) - 1) {
+      base[q] = atomicAdd(&d.cellCount[k[q]], (uint32_t)__popc(peers[q]));
       // this substep's per-cell displacement slots start at zero for every occupied
       // cell (list reuse only: a slot left larger makes the bound looser, never wrong).
       // Done here by the warp leaders rather than in the scan: measured cheaper, the
@@ -49,36 +61,54 @@ __device__ __forceinline__ void key_count_body(const SimParams& P, const DevScen
       // ~60 us per launch on the 96-scene mix and saved ~6 us here).
       if (d.cellDisp) {
         const uint32_t slots = min(P.iters, (uint32_t)kDispSlots);
-        for (uint32_t t = 0; t < slots; t++) d.cellDisp[(size_t)t * d.cellStride + k] = 0.0f;
+        for (uint32_t t = 0; t < slots; t++) d.cellDisp[(size_t)t * d.cellStride + k[q]] = 0.0f;
       }
     }
-    base = __shfl_sync(peers, base, leader);
-    d.key[i] = k;
-    d.rank[i] = base + (uint32_t)__popc(lt);
+  }
+#pragma unroll
+  for (int q = 0; q < N; q++) {
+    base[q] = __shfl_sync(0xffffffffu, base[q], __ffs(peers[q]) - 1);
+    if (k[q] != 0xffffffffu) {
+      const uint32_t i = P.pOff + li + q * step;
+      d.key[i] = k[q];
+      d.rank[i] = base[q] + (uint32_t)__popc(peers[q] & ((1u << lane) - 1u));
+    }
   }
 }
 
-__device__ __forceinline__ void fill_body(const SimParams& P, const DevScene& d, uint32_t li) {
-  if (li >= P.n) return;
-  const uint32_t i = P.pOff + li;
-  const uint32_t at = __ldg(&d.cellStart[d.key[i]]) + d.rank[i];
-  if (at < P.pEnd) d.unordered[at] = i;  // always true after a completed scan
+template <int N>
+__device__ __forceinline__ void fill_body(const SimParams& P, const DevScene& d, uint32_t li, uint32_t step) {
+  uint32_t at[N];
+#pragma unroll
+  for (int q = 0; q < N; q++) {
+    const uint32_t i = P.pOff + li + q * step;
+    at[q] = P.pEnd;
+    if (li + q * step < P.n) at[q] = __ldg(&d.cellStart[d.key[i]]) + d.rank[i];
+  }
+#pragma unroll
+  for (int q = 0; q < N; q++)
+    if (at[q] < P.pEnd) d.unordered[at[q]] = P.pOff + li + q * step;  // always, after a completed scan
 }
 
+// Takes the particle in place li of the unordered buckets to its place in the stable
+// order, which is in the same bucket: a warp's reads then come from wherever its
+// particles were and its writes fall into a few whole lines. (Read in the old order and
+// scattered into the new, the half-sector writes were the cost: 73 us for 1,000,003
+// particles shuffled within 600 places, against 50 us.)
 __device__ __forceinline__ void reorder_body(const SimParams& P, const DevScene& d, uint32_t li) {
   if (li >= P.n) return;
-  const uint32_t i = P.pOff + li;
   const int src = P.parity, dst = P.parity ^ 1;
+  // min() and max() keep every access in bounds even if a scan gave up (error word set)
+  const uint32_t i = max(min(d.unordered[P.pOff + li], P.pEnd - 1u), P.pOff);
+  const float4 p4 = __ldg(&d.pos[src][i]), v4 = __ldg(&d.vel[src][i]);
   const uint32_t k = d.key[i];
-  // min() keeps every access in bounds even if a scan gave up (error word set)
   const uint32_t e = min(__ldg(&d.cellStart[k + 1]), P.pEnd);
   const uint32_t b = min(__ldg(&d.cellStart[k]), e);
   uint32_t r = 0;
   for (uint32_t m = b; m < e; m++) r += __ldg(&d.unordered[m]) < i ? 1u : 0u;
   const uint32_t s = min(b + r, P.pEnd - 1u);
-  const float4 p4 = __ldg(&d.pos[src][i]);
   F3 v, pr;
-  predict_one(P, p4, __ldg(&d.vel[src][i]), v, pr);
+  predict_one(P, p4, v4, v, pr);
   d.pos[dst][s] = p4;
   d.vel[dst][s] = make_float4(v.x, v.y, v.z, 0.0f);
   d.pred[dst][s] = make_float4(pr.x, pr.y, pr.z, 1.0f);
@@ -93,27 +123,29 @@ __device__ __forceinline__ void reorder_body(const SimParams& P, const DevScene&
     }
   }
   if (d.rest[src]) d.rest[dst][s] = __ldg(&d.rest[src][i]);
-  if (d.slotOut) d.slotOut[li] = s - P.pOff;
+  if (d.slotOut) d.slotOut[i - P.pOff] = s - P.pOff;
 }
 
+template <int N>
 __global__ void __launch_bounds__(kBlock) k_key_count(const __grid_constant__ SimParams P,
                                                       const __grid_constant__ DevScene d) {
-  key_count_body(P, d, blockIdx.x * kBlock + threadIdx.x);
+  key_count_body<N>(P, d, blockIdx.x * (kBlock * N) + threadIdx.x, kBlock);
 }
 // The batched streaming passes take whole 256-particle tiles per claim (one atomic
 // per tile instead of one per 32-particle slice: their per-particle work is short,
 // so a cursor shared by every warp would serialise them).
 __global__ void __launch_bounds__(kBlock) k_key_count_b(const __grid_constant__ BatchWork w,
                                                         const __grid_constant__ DevScene d) {
-  for_each_item(w, [&](const SimParams& P, uint32_t t, uint32_t) { key_count_body(P, d, t * kBlock + threadIdx.x); });
+  for_each_item(w, [&](const SimParams& P, uint32_t t, uint32_t) { key_count_body<1>(P, d, t * kBlock + threadIdx.x, 0u); });
 }
+template <int N>
 __global__ void __launch_bounds__(kBlock) k_fill(const __grid_constant__ SimParams P,
                                                  const __grid_constant__ DevScene d) {
-  fill_body(P, d, blockIdx.x * kBlock + threadIdx.x);
+  fill_body<N>(P, d, blockIdx.x * (kBlock * N) + threadIdx.x, kBlock);
 }
 __global__ void __launch_bounds__(kBlock) k_fill_b(const __grid_constant__ BatchWork w,
                                                    const __grid_constant__ DevScene d) {
-  for_each_item(w, [&](const SimParams& P, uint32_t t, uint32_t) { fill_body(P, d, t * kBlock + threadIdx.x); });
+  for_each_item(w, [&](const SimParams& P, uint32_t t, uint32_t) { fill_body<1>(P, d, t * kBlock + threadIdx.x, 0u); });
 }
 __global__ void __launch_bounds__(kBlock) k_reorder(const __grid_constant__ SimParams P,
                                                     const __grid_constant__ DevScene d) {
@@ -154,17 +186,23 @@ __device__ __forceinline__ void scan_tile(uint32_t* __restrict__ cellCount,
   const long long base = cellBase + (long long)tid * kScanItems;
   uint32_t v[kScanItems];
   uint32_t sum = 0;
+  // eight counts as two 16-byte words; a caller's workspace may be aligned to less
+  const bool whole = base + kScanItems <= limit && (reinterpret_cast<uintptr_t>(cellCount) & 15u) == 0u;
+  if (whole) {
+    uint4* c = reinterpret_cast<uint4*>(cellCount + base);
+    const uint4 a = c[0], b = c[1];
+    c[0] = c[1] = make_uint4(0u, 0u, 0u, 0u);
+    v[0] = a.x; v[1] = a.y; v[2] = a.z; v[3] = a.w;
+    v[4] = b.x; v[5] = b.y; v[6] = b.z; v[7] = b.w;
+  } else {
 #pragma unroll
-  for (int j = 0; j < kScanItems; j++) {
-    const long long idx = base + j;
-    v[j] = idx < limit ? cellCount[idx] : 0u;
-    sum += v[j];
+    for (int j = 0; j < kScanItems; j++) {
+      v[j] = base + j < limit ? cellCount[base + j] : 0u;
+      if (base + j < limit) cellCount[base + j] = 0u;
+    }
   }
 #pragma unroll
-  for (int j = 0; j < kScanItems; j++) {
-    const long long idx = base + j;
-    if (idx < limit) cellCount[idx] = 0u;
-  }
+  for (int j = 0; j < kScanItems; j++) sum += v[j];
   uint32_t incl = sum;
 #pragma unroll
   for (int o = 1; o < 32; o <<= 1) {
@@ -377,9 +415,16 @@ __global__ void __launch_bounds__(kBlock) k_scan_apply_b(const __grid_constant__
   });
 }
 
+// From here on one particle per thread no longer fits the GPU at once (2,048 threads on
+// each of 148 SMs), and four per thread keep more loads and atomics in flight: key 27 ->
+// 20 us and fill 12.3 -> 11.2 us for 1,000,003 shuffled particles, 12.4 -> 10.0 us for
+// the fill of the large scene.
+constexpr uint32_t kManyParticles = 300000u;
+
 void launch_key_count(const SimParams& P, const DevScene& d, cudaStream_t st) {
   const long long work = (long long)P.n > (long long)P.nBodies ? P.n : P.nBodies;
-  k_key_count<<<groups(work), kBlock, 0, st>>>(P, d);
+  if (P.n >= kManyParticles) k_key_count<4><<<groups(work, 4 * kBlock), kBlock, 0, st>>>(P, d);
+  else k_key_count<1><<<groups(work), kBlock, 0, st>>>(P, d);
 }
 void launch_scan(uint32_t* cellCount, uint32_t* cellStart, int nCells, unsigned long long* state,
                  uint32_t* ticket, uint32_t epoch, uint32_t* err, cudaStream_t st, uint32_t spinLimit) {
@@ -387,7 +432,8 @@ void launch_scan(uint32_t* cellCount, uint32_t* cellStart, int nCells, unsigned 
   k_scan<<<tiles, kBlock, 0, st>>>(cellCount, cellStart, nCells, state, ticket, epoch, tiles, err, spinLimit);
 }
 void launch_fill(const SimParams& P, const DevScene& d, cudaStream_t st) {
-  k_fill<<<groups(P.n), kBlock, 0, st>>>(P, d);
+  if (P.n >= kManyParticles) k_fill<4><<<groups(P.n, 4 * kBlock), kBlock, 0, st>>>(P, d);
+  else k_fill<1><<<groups(P.n), kBlock, 0, st>>>(P, d);
 }
 void launch_reorder(const SimParams& P, const DevScene& d, cudaStream_t st) {
   k_reorder<<<groups(P.n), kBlock, 0, st>>>(P, d);
