@@ -299,6 +299,22 @@ void pack_params(p4a_sim* s, double dt) {
   F.pairMath = pair_math_ranges(F);
 }
 
+// Lanes per particle of the neighbour passes of a plain scene (0: one thread per
+// particle). A group shortens each particle's chain of dependent loads but issues more
+// instructions, so it gains while the GPU has idle schedulers, also with other scenes on
+// other streams. us per frame, one scene alone / a frame of three scenes on three streams,
+// with one thread, 16 and 8 lanes per particle, dam break (D, 2 substeps of 4 iterations)
+// and the sloshing preset (P, 4 of 4, lists rebuilt in most iterations):
+//   D  2,197: 309/125 187/86  192/89      P  2,500: 1397/558  597/252  638/271
+//   D  4,000: 342/137 201/94  212/93      P  5,000: 1448/592  640/280  673/292
+//   D  8,000: 356/145 225/109 230/105     P  8,000: 1479/603  683/331  716/318
+//   D 16,000: 376/156 293/149 257/133     P 16,000: 1494/629  963/502  822/435
+//   D 24,000: 387/162 356/197 326/172     P 24,000: 1604/673 1162/691 1083/593
+//   D 32,768: 392/169 415/255 362/214     P 40,000: 1713/774 1593/1093 1411/911
+// Past 20,000 particles the lone scene still gains but scenes side by side lose.
+constexpr int kGroup16 = 6000, kGroup8 = 20000;
+int group_lanes(int n) { return n <= kGroup16 ? 16 : n <= kGroup8 ? 8 : 0; }
+
 uint32_t next_epoch(p4a_sim* s) {
   s->scanEpoch = (s->scanEpoch + 1) & 0x3fffffffu;
   if (s->scanEpoch == 0) s->scanEpoch = 1;
@@ -827,6 +843,7 @@ int p4a_step(p4a_sim* s, double frameDt, int32_t* substeps_out) {
   const float goal[3] = {(float)s->heldTarget[0], (float)s->heldTarget[1], (float)s->heldTarget[2]};
   const int iters = std::max(1, p.iterations);
   const bool tension = p.surface_tension_k > 0;
+  const int G = group_lanes(s->n);
   for (int step = 0; step < sub; step++) {
     const int par = s->parity, q = par ^ 1;
     if (dragging) {
@@ -845,9 +862,11 @@ int p4a_step(p4a_sim* s, double frameDt, int32_t* substeps_out) {
     }
     for (int it = 0; it < iters; it++) {
       mark(s, PH_LAMBDA);
-      launch_lambda(P, d, it, st);
+      if (G) launch_lambda_g(P, d, it, G, st);
+      else launch_lambda(P, d, it, st);
       mark(s, PH_DELTA);
-      launch_delta(P, d, it, st);
+      if (G) launch_delta_g(P, d, it, G, st);
+      else launch_delta(P, d, it, st);
       if (bodies) {
         mark(s, PH_BODY_MATCH);
         launch_body_match(P, d, it, st);
@@ -859,12 +878,19 @@ int p4a_step(p4a_sim* s, double frameDt, int32_t* substeps_out) {
     }
     if (tension) {
       mark(s, PH_XSPH_NORMALS);
-      launch_xsph_normals(P, d, st);
+      if (G) launch_xsph_normals_g(P, d, G, st);
+      else launch_xsph_normals(P, d, st);
       mark(s, PH_TENSION_FINALIZE);
-      launch_tension_finalize(P, d, step, st);
+      if (G) launch_tension_finalize_g(P, d, G, st);
+      else launch_tension_finalize(P, d, step, st);
     } else {
       mark(s, PH_XSPH_FINALIZE);
-      launch_xsph_finalize(P, d, step, st);
+      if (G) launch_xsph_finalize_g(P, d, G, st);
+      else launch_xsph_finalize(P, d, step, st);
+    }
+    if (G && step == sub - 1) {
+      count_launches(1);
+      launch_stats(P, d, st);
     }
     s->simTime += dt;
   }

@@ -338,6 +338,19 @@ __global__ void __launch_bounds__(kBlock, kTensionBlocksBatched) k_tension_final
   for_each_item(w, [&](const SimParams& P, uint32_t t, uint32_t) { tension_finalize_body(P, d, t, substep); });
 }
 
+// The stats pass on its own, for the group passes (kernels_group.cu), whose blocks are no
+// tiles of 256 particles: the same trees over the stored densities and velocities.
+__global__ void __launch_bounds__(kBlock) k_stats(const __grid_constant__ SimParams P,
+                                                  const __grid_constant__ DevScene d) {
+  const uint32_t li = blockIdx.x * kBlock + threadIdx.x;
+  const bool act = li < P.n;
+  const uint32_t i = P.pOff + (act ? li : 0u);
+  block_stats(P, act, __ldg(&d.density[i]), xyz(__ldg(&d.vel[(int)P.parity ^ 1][i])), d.statsOut + 8 * P.slot);
+}
+void launch_stats(const SimParams& P, const DevScene& d, cudaStream_t st) {
+  k_stats<<<groups(P.n), kBlock, 0, st>>>(P, d);
+}
+
 void launch_xsph_finalize(const SimParams& P, const DevScene& d, int substep, cudaStream_t st) {
   k_xsph_finalize<<<groups(P.n), kBlock, 0, st>>>(P, d, substep);
 }

@@ -217,7 +217,6 @@ __device__ __forceinline__ void delta_body(const SimParams& P, const DevScene& d
   if (li >= P.n) return;
   const uint32_t i = P.pOff + li;
   const int L = (int)P.parity ^ 1;
-  float4* __restrict__ predOut = d.pred[L ^ ((it + 1) & 1)];
   // lambda's (position, lambda) of this iteration: the positions of pred[L ^ (it & 1)]
   const float4* __restrict__ pl = d.predLam;
   const float4 self = __ldg(&pl[i]);
@@ -267,25 +266,7 @@ __device__ __forceinline__ void delta_body(const SimParams& P, const DevScene& d
       walk_direct<true>(P, w, pi, i, pl, d.cellStart + P.cOff, d.bcellStart + P.cOff, d.bsample, fluid, bound);
     }
   }
-  const F3 dd = {fmaf(dB.x, P.invRho0, dsum.x * P.volume), fmaf(dB.y, P.invRho0, dsum.y * P.volume),
-                 fmaf(dB.z, P.invRho0, dsum.z * P.volume)};
-  float scale = P.omega;
-  if (P.sorAverage == 1u) scale = P.omega / fmaxf(nc, 1.0f);
-  F3 o = fma3(scale, dd, pi);
-  o.x = fminf(fmaxf(o.x, P.clampMin[0]), P.clampMax[0]);
-  o.y = fminf(fmaxf(o.y, P.clampMin[1]), P.clampMax[1]);
-  o.z = fminf(fmaxf(o.z, P.clampMin[2]), P.clampMax[2]);
-  predOut[i] = make_float4(o.x, o.y, o.z, 1.0f);
-  if (it < kDispSlots) {
-    record_displacement(d, P, it, sub3(o, pi));
-    record_cell_displacement(d, P, it, o, xyz(__ldg(&d.nbRef[i])));
-  }
-  if (it == (int)P.iters - 1) {  // velFromPos into the non-live velocity copy
-    const float4 p0 = __ldg(&d.pos[L][i]);
-    const F3 v = {(o.x - p0.x) * P.invDt, (o.y - p0.y) * P.invDt, (o.z - p0.z) * P.invDt};
-    d.vel[L ^ 1][i] = make_float4(v.x, v.y, v.z, 0.0f);
-    d.velRho[i] = make_float4(v.x, v.y, v.z, fmaxf(__ldg(&d.density[i]), 0.5f * P.rho0));
-  }
+  delta_finish(P, d, i, it, L, pi, dsum, dB, nc);
 }
 
 // Plain: block b handles particles [b * TB, (b + 1) * TB). Batched: warps pull

@@ -338,6 +338,16 @@ void launch_xsph_finalize(const SimParams& P, const DevScene& d, int substep, cu
 void launch_xsph_normals(const SimParams& P, const DevScene& d, cudaStream_t st, int variant = -1);
 void launch_tension_finalize(const SimParams& P, const DevScene& d, int substep, cudaStream_t st);
 
+// The same passes with a group of G = 8 or 16 lanes per particle (kernels_group.cu)
+// for scenes too small to fill the GPU with one thread per particle; the stats are a
+// launch of their own after the last substep's finalize.
+void launch_lambda_g(const SimParams& P, const DevScene& d, int it, int G, cudaStream_t st);
+void launch_delta_g(const SimParams& P, const DevScene& d, int it, int G, cudaStream_t st);
+void launch_xsph_finalize_g(const SimParams& P, const DevScene& d, int G, cudaStream_t st);
+void launch_xsph_normals_g(const SimParams& P, const DevScene& d, int G, cudaStream_t st);
+void launch_tension_finalize_g(const SimParams& P, const DevScene& d, int G, cudaStream_t st);
+void launch_stats(const SimParams& P, const DevScene& d, cudaStream_t st);
+
 // ---- batched launchers (items: tiles of 256 particles, scan tiles, or bodies) ----
 // `maxItems` bounds the launch's item count: the grid is min(maxItems, the blocks
 // resident on the device at once); pass a large value for a launch whose count is

@@ -93,4 +93,21 @@ __device__ __forceinline__ F2 quot2(F2 a, F2 s, F2 yn) {
   return fma2(fma2(s, qn, a), yn, qn);
 }
 
+// The same for one pair: s = sqrt(x) rounded, -1 / s, -1 / d, and a / s.
+struct Root1 {
+  float s, yn;
+};
+__device__ __forceinline__ Root1 root1(float x) {
+  const float y = rsqrt_approx(x), g = x * y, s = fmaf(fmaf(-g, g, x), 0.5f * y, g), yn = y * kOneUp;
+  return {s, fmaf(fmaf(s, yn, 1.0f), yn, yn)};
+}
+__device__ __forceinline__ float recip1(float d) {
+  const float y = rcp_approx(d);
+  return fmaf(fmaf(d, y, -1.0f), y, -y);
+}
+__device__ __forceinline__ float quot1(float a, float s, float yn) {
+  const float qn = a * yn;
+  return -fmaf(fmaf(s, qn, a), yn, qn);
+}
+
 }  // namespace p4a
