@@ -6,9 +6,9 @@
 //   body_match  the per-iteration chain bodyClear, bodyCentre, bodySeed, bodyCov,
 //               bodyResolve, bodyProject
 // The sums are the reference's fixed-point i32 values (round half to even of
-// (pred - centre) * bodyScale and of p_r q_c * covScale), added with wrap-around
-// in a warp-shuffle tree: integer addition is associative, so the totals are the
-// bits the reference's atomics produce in any order. The resolve runs on one
+// (pred - centre) * bodyScale and of p_r q_c * covScale), added with wrap-around:
+// integer addition is associative, so the totals are the bits the reference's
+// atomics produce in any order. The resolve runs on one
 // thread with the reference's float order.
 // The per-body particle lists are rebuilt by the reorder of every sort
 // (bodyList[bodyStart[b] + k]), replacing the reference's global atomic compaction.
@@ -23,58 +23,71 @@
 
 namespace p4a {
 
-constexpr int kBodyBlock = 256;
+// A body's match is one block's chain of dependent steps (particle list, gathers, two
+// sums, the resolve on one thread, the projection), so it is bound by latency: a thread
+// keeps index, positions and rest offset of its first K particles in registers through
+// all steps, loaded together, and only bodies of more than TB * K particles read the rest
+// again in each step; a sum is one reduction instruction per warp and term, and every
+// warp adds up the warps' sums for itself. One launch with its event, three bodies of 736
+// to 1,089 particles / 8 of 216 / 64 of 32 to 1,000: 18.8 / 12.2 / 23.1 us with 256
+// threads that read the list in each step, 14.4 / 10.5 / 12.6 us as it is. In a batch the
+// blocks of 48 and more scenes fill the GPU and smaller ones pack better: 96 mixed scenes
+// 16.2 us with 256 x 4, 18.8 us with 512 x 2.
+constexpr int kBodyBlock = 512, kBodyHeld = 2;             // one scene
+constexpr int kBodyBlockBatched = 256, kBodyHeldBatched = 4;
 
-__device__ __forceinline__ uint32_t warp_sum_u32(uint32_t v) {
-#pragma unroll
-  for (int o = 16; o > 0; o >>= 1) v += __shfl_xor_sync(0xffffffffu, v, o);
-  return v;
-}
-
-// Sum N u32 lanes over the block; result valid in s_out[0..N) after the call.
-template <int N>
-__device__ __forceinline__ void block_sum_u32(uint32_t (&v)[N], uint32_t* s_scratch,
-                                              uint32_t* s_out) {
+// Sum N u32 lanes over the block; every lane of every warp gets the totals. `s` holds
+// N * 32 words and is not reused without a barrier in between.
+template <int TB, int N>
+__device__ __forceinline__ void block_sum_u32(uint32_t (&v)[N], uint32_t* s) {
   const int lane = threadIdx.x & 31, warp = threadIdx.x >> 5;
 #pragma unroll
   for (int k = 0; k < N; k++) {
-    const uint32_t w = warp_sum_u32(v[k]);
-    if (lane == 0) s_scratch[warp * N + k] = w;
+    const uint32_t w = __reduce_add_sync(0xffffffffu, v[k]);
+    if (lane == 0) s[k * 32 + warp] = w;
   }
   __syncthreads();
-  if (threadIdx.x < N) {
-    uint32_t t = 0;
-    for (int w = 0; w < kBodyBlock / 32; w++) t += s_scratch[w * N + threadIdx.x];
-    s_out[threadIdx.x] = t;
-  }
-  __syncthreads();
+#pragma unroll
+  for (int k = 0; k < N; k++)
+    v[k] = __reduce_add_sync(0xffffffffu, lane < TB / 32 ? s[k * 32 + lane] : 0u);
 }
 
-// acc = sum round((pred - centre) * bodyScale) over the body (bodyCentre pass).
-__device__ __forceinline__ void centre_sums(const SimParams& P, const float4* __restrict__ pred,
-                                            const uint32_t* __restrict__ list, uint32_t count,
-                                            F3 centre, uint32_t* s_scratch, uint32_t* s_acc) {
-  uint32_t a[3] = {0u, 0u, 0u};
-  for (uint32_t t = threadIdx.x; t < count; t += kBodyBlock) {
-    const uint32_t i = list[t];
-    const F3 d = mul3(sub3(xyz(pred[i]), centre), P.bodyScale);
-    a[0] += (uint32_t)round_i32(d.x);
-    a[1] += (uint32_t)round_i32(d.y);
-    a[2] += (uint32_t)round_i32(d.z);
-  }
-  block_sum_u32<3>(a, s_scratch, s_acc);
+// A term of acc = sum round((pred - centre) * bodyScale) over the body (bodyCentre pass).
+__device__ __forceinline__ void add_centre(const SimParams& P, F3 p, F3 centre, uint32_t (&a)[3]) {
+  const F3 d = mul3(sub3(p, centre), P.bodyScale);
+  a[0] += (uint32_t)round_i32(d.x);
+  a[1] += (uint32_t)round_i32(d.y);
+  a[2] += (uint32_t)round_i32(d.z);
 }
 
+// A term of A = sum round((pred - ref)_r * rest_c * covScale), column-major (bodyCov).
+__device__ __forceinline__ void add_cov(const SimParams& P, F3 pos, F3 ref, F3 q, uint32_t (&cv)[9]) {
+  const F3 p = sub3(pos, ref);
+  cv[0] += (uint32_t)round_i32(p.x * q.x * P.covScale);
+  cv[1] += (uint32_t)round_i32(p.y * q.x * P.covScale);
+  cv[2] += (uint32_t)round_i32(p.z * q.x * P.covScale);
+  cv[3] += (uint32_t)round_i32(p.x * q.y * P.covScale);
+  cv[4] += (uint32_t)round_i32(p.y * q.y * P.covScale);
+  cv[5] += (uint32_t)round_i32(p.z * q.y * P.covScale);
+  cv[6] += (uint32_t)round_i32(p.x * q.z * P.covScale);
+  cv[7] += (uint32_t)round_i32(p.y * q.z * P.covScale);
+  cv[8] += (uint32_t)round_i32(p.z * q.z * P.covScale);
+}
+
+template <int TB, int K>
 __device__ __forceinline__ void body_seed_body(const SimParams& P, const DevScene& d, uint32_t b) {
-  __shared__ uint32_t s_scratch[(kBodyBlock / 32) * 9];
-  __shared__ uint32_t s_acc[9];
+  __shared__ uint32_t s_sum[3 * 32];
   const uint32_t gb = P.bOff + b;
   const float4* __restrict__ pred = d.pred[(int)P.parity ^ 1];
   const uint32_t start = d.bodyStart[gb], count = d.bodyStart[gb + 1] - start;
+  const uint32_t* __restrict__ list = d.bodyList + start;
   const F3 centre = xyz(d.bodyCentre[gb]);
-  centre_sums(P, pred, d.bodyList + start, count, centre, s_scratch, s_acc);
+  uint32_t a[3] = {0u, 0u, 0u};
+#pragma unroll K
+  for (uint32_t t = threadIdx.x; t < count; t += TB) add_centre(P, xyz(pred[list[t]]), centre, a);
+  block_sum_u32<TB, 3>(a, s_sum);
   if (threadIdx.x == 0) {
-    const int32_t ax = (int32_t)s_acc[0], ay = (int32_t)s_acc[1], az = (int32_t)s_acc[2];
+    const int32_t ax = (int32_t)a[0], ay = (int32_t)a[1], az = (int32_t)a[2];
     d.bodyAccum[gb * 4 + 0] = ax; d.bodyAccum[gb * 4 + 1] = ay; d.bodyAccum[gb * 4 + 2] = az;
     d.bodyAccum[gb * 4 + 3] = (int32_t)count;
 #pragma unroll
@@ -98,64 +111,75 @@ __device__ __forceinline__ M3 inverse_transposed(const M3& m) {
   return {{mul3(r0, invd), mul3(r1, invd), mul3(r2, invd)}};
 }
 
+template <int TB, int K>
 __device__ __forceinline__ void body_match_body(const SimParams& P, const DevScene& d, uint32_t b, int it) {
-  __shared__ uint32_t s_scratch[(kBodyBlock / 32) * 9];
-  __shared__ uint32_t s_acc[9];
-  __shared__ float s_ref[3];
+  __shared__ uint32_t s_sum[(3 + 9) * 32];
   __shared__ float s_pose[12];  // centre xyz, rows of R
   const int L = (int)P.parity ^ 1;
   float4* __restrict__ pred = d.pred[L ^ ((it + 1) & 1)];
   const float4* __restrict__ rest = d.rest[L];
   const uint32_t gb = P.bOff + b;
   const uint32_t start = d.bodyStart[gb], count = d.bodyStart[gb + 1] - start;
-  const uint32_t* list = d.bodyList + start;
+  const uint32_t* __restrict__ list = d.bodyList + start;
   const F3 centre = xyz(d.bodyCentre[gb]);
+  F3 refOld = xyz(d.bodyRef[gb]);
+  const bool moves = it < kDispSlots;
+  // the thread's first particles, all loads in flight at once
+  uint32_t hi[K];
+  F3 hp[K], hq[K], hFrom[K], hRef[K];
+#pragma unroll
+  for (int k = 0; k < K; k++) {
+    const uint32_t t = threadIdx.x + (uint32_t)k * TB;
+    hi[k] = t < count ? list[t] : 0xffffffffu;
+  }
+#pragma unroll
+  for (int k = 0; k < K; k++) {
+    const bool has = hi[k] != 0xffffffffu;
+    const F3 zero = {0.f, 0.f, 0.f};
+    hp[k] = has ? xyz(pred[hi[k]]) : zero;
+    hq[k] = has ? xyz(__ldg(&rest[hi[k]])) : zero;
+    hFrom[k] = has && moves ? xyz(__ldg(&d.pred[L ^ (it & 1)][hi[k]])) : zero;
+    hRef[k] = has && moves ? xyz(__ldg(&d.nbRef[hi[k]])) : zero;
+  }
   // bodyClear + bodyCentre
-  centre_sums(P, pred, list, count, centre, s_scratch, s_acc);
-  const int32_t ax = (int32_t)s_acc[0], ay = (int32_t)s_acc[1], az = (int32_t)s_acc[2];
+  uint32_t a[3] = {0u, 0u, 0u};
+#pragma unroll
+  for (int k = 0; k < K; k++)
+    if (hi[k] != 0xffffffffu) add_centre(P, hp[k], centre, a);
+  for (uint32_t t = threadIdx.x + K * TB; t < count; t += TB)
+    add_centre(P, xyz(pred[list[t]]), centre, a);
+  block_sum_u32<TB, 3>(a, s_sum);
+  const int32_t ax = (int32_t)a[0], ay = (int32_t)a[1], az = (int32_t)a[2];
   const float cnt = (float)(int32_t)count;
-  // bodySeed: bodyRef = bodyCentre + mean offset
-  if (threadIdx.x == 0) {
-    F3 r = xyz(d.bodyRef[gb]);
-    if (cnt > 0.0f) {
-      const float den = P.bodyScale * cnt;
-      r = {centre.x + (float)ax / den, centre.y + (float)ay / den, centre.z + (float)az / den};
-      d.bodyRef[gb] = make_float4(r.x, r.y, r.z, 0.0f);
-    }
-    s_ref[0] = r.x; s_ref[1] = r.y; s_ref[2] = r.z;
+  const float den = P.bodyScale * cnt;
+  // bodySeed: bodyRef = bodyCentre + mean offset, by every thread
+  F3 delta = {0.f, 0.f, 0.f}, ref = refOld;
+  if (cnt > 0.0f) {
+    delta = {(float)ax / den, (float)ay / den, (float)az / den};
+    ref = {centre.x + delta.x, centre.y + delta.y, centre.z + delta.z};
+    if (threadIdx.x == 0) d.bodyRef[gb] = make_float4(ref.x, ref.y, ref.z, 0.0f);
   }
-  __syncthreads();
-  // bodyCov: A = sum round((pred - ref)_r * rest_c * covScale), column-major
-  const F3 ref = {s_ref[0], s_ref[1], s_ref[2]};
+  // bodyCov
   uint32_t cv[9] = {0u, 0u, 0u, 0u, 0u, 0u, 0u, 0u, 0u};
-  for (uint32_t t = threadIdx.x; t < count; t += kBodyBlock) {
+#pragma unroll
+  for (int k = 0; k < K; k++)
+    if (hi[k] != 0xffffffffu) add_cov(P, hp[k], ref, hq[k], cv);
+  for (uint32_t t = threadIdx.x + K * TB; t < count; t += TB) {
     const uint32_t i = list[t];
-    const F3 p = sub3(xyz(pred[i]), ref);
-    const F3 q = xyz(__ldg(&rest[i]));
-    cv[0] += (uint32_t)round_i32(p.x * q.x * P.covScale);
-    cv[1] += (uint32_t)round_i32(p.y * q.x * P.covScale);
-    cv[2] += (uint32_t)round_i32(p.z * q.x * P.covScale);
-    cv[3] += (uint32_t)round_i32(p.x * q.y * P.covScale);
-    cv[4] += (uint32_t)round_i32(p.y * q.y * P.covScale);
-    cv[5] += (uint32_t)round_i32(p.z * q.y * P.covScale);
-    cv[6] += (uint32_t)round_i32(p.x * q.z * P.covScale);
-    cv[7] += (uint32_t)round_i32(p.y * q.z * P.covScale);
-    cv[8] += (uint32_t)round_i32(p.z * q.z * P.covScale);
+    add_cov(P, xyz(pred[i]), ref, xyz(__ldg(&rest[i])), cv);
   }
-  block_sum_u32<9>(cv, s_scratch, s_acc);
+  block_sum_u32<TB, 9>(cv, s_sum + 3 * 32);
   // bodyResolve on one thread
   if (threadIdx.x == 0) {
     d.bodyAccum[gb * 4 + 0] = ax; d.bodyAccum[gb * 4 + 1] = ay; d.bodyAccum[gb * 4 + 2] = az;
     d.bodyAccum[gb * 4 + 3] = (int32_t)count;
     int32_t c9[9];
 #pragma unroll
-    for (int k = 0; k < 9; k++) { c9[k] = (int32_t)s_acc[k]; d.bodyCov[gb * 9 + k] = c9[k]; }
+    for (int k = 0; k < 9; k++) { c9[k] = (int32_t)cv[k]; d.bodyCov[gb * 9 + k] = c9[k]; }
     F3 cen = centre;
     float rows[9];
     bool wrote = false;
     if (cnt > 0.0f) {
-      const float den = P.bodyScale * cnt;
-      F3 delta = {(float)ax / den, (float)ay / den, (float)az / den};
       const float invRatio = d.bodyInfo[gb].x;
       if (invRatio > 0.0f) delta = mul3(delta, invRatio);
       cen = {centre.x + delta.x, centre.y + delta.y, centre.z + delta.z};
@@ -204,16 +228,14 @@ __device__ __forceinline__ void body_match_body(const SimParams& P, const DevSce
   const F3 cen = {s_pose[0], s_pose[1], s_pose[2]};
   const F3 r0 = {s_pose[3], s_pose[4], s_pose[5]}, r1 = {s_pose[6], s_pose[7], s_pose[8]},
            r2 = {s_pose[9], s_pose[10], s_pose[11]};
-  for (uint32_t t = threadIdx.x; t < count; t += kBodyBlock) {
-    const uint32_t i = list[t];
-    const F3 q = xyz(__ldg(&rest[i]));
+  // the projection moves the particle from this iteration's input position `from`
+  auto project = [&](uint32_t i, F3 q, F3 from, F3 start0) {
     const F3 p = {dot3(r0, q), dot3(r1, q), dot3(r2, q)};
     const F3 o = add3(cen, p);
     pred[i] = make_float4(o.x, o.y, o.z, 1.0f);
-    // the projection moves the particle from this iteration's input position
-    if (it < kDispSlots) {
-      record_displacement(d, P, it, sub3(o, xyz(__ldg(&d.pred[L ^ (it & 1)][i]))));
-      record_cell_displacement(d, P, it, o, xyz(__ldg(&d.nbRef[i])));
+    if (moves) {
+      record_displacement(d, P, it, sub3(o, from));
+      record_cell_displacement(d, P, it, o, start0);
     }
     if (last) {
       const float4 p0 = __ldg(&d.pos[L][i]);
@@ -221,25 +243,38 @@ __device__ __forceinline__ void body_match_body(const SimParams& P, const DevSce
       d.vel[L ^ 1][i] = make_float4(v.x, v.y, v.z, 0.0f);
       d.velRho[i] = make_float4(v.x, v.y, v.z, fmaxf(__ldg(&d.density[i]), 0.5f * P.rho0));
     }
+  };
+#pragma unroll
+  for (int k = 0; k < K; k++)
+    if (hi[k] != 0xffffffffu) project(hi[k], hq[k], hFrom[k], hRef[k]);
+  for (uint32_t t = threadIdx.x + K * TB; t < count; t += TB) {
+    const uint32_t i = list[t];
+    const F3 zero = {0.f, 0.f, 0.f};
+    project(i, xyz(__ldg(&rest[i])), moves ? xyz(__ldg(&d.pred[L ^ (it & 1)][i])) : zero,
+            moves ? xyz(__ldg(&d.nbRef[i])) : zero);
   }
 }
 
 __global__ void __launch_bounds__(kBodyBlock) k_body_seed(const __grid_constant__ SimParams P,
                                                           const __grid_constant__ DevScene d) {
-  body_seed_body(P, d, blockIdx.x);
+  body_seed_body<kBodyBlock, kBodyHeld>(P, d, blockIdx.x);
 }
-__global__ void __launch_bounds__(kBodyBlock) k_body_seed_b(const __grid_constant__ BatchWork w,
-                                                            const __grid_constant__ DevScene d) {
-  for_each_item(w, [&](const SimParams& P, uint32_t t, uint32_t) { body_seed_body(P, d, t); });
+__global__ void __launch_bounds__(kBodyBlockBatched) k_body_seed_b(const __grid_constant__ BatchWork w,
+                                                                   const __grid_constant__ DevScene d) {
+  for_each_item(w, [&](const SimParams& P, uint32_t t, uint32_t) {
+    body_seed_body<kBodyBlockBatched, kBodyHeldBatched>(P, d, t);
+  });
 }
 __global__ void __launch_bounds__(kBodyBlock) k_body_match(const __grid_constant__ SimParams P,
                                                            const __grid_constant__ DevScene d, int it) {
-  body_match_body(P, d, blockIdx.x, it);
+  body_match_body<kBodyBlock, kBodyHeld>(P, d, blockIdx.x, it);
 }
-__global__ void __launch_bounds__(kBodyBlock) k_body_match_b(const __grid_constant__ BatchWork w,
-                                                             const __grid_constant__ DevScene d,
-                                                             int it) {
-  for_each_item(w, [&](const SimParams& P, uint32_t t, uint32_t) { body_match_body(P, d, t, it); });
+__global__ void __launch_bounds__(kBodyBlockBatched) k_body_match_b(const __grid_constant__ BatchWork w,
+                                                                    const __grid_constant__ DevScene d,
+                                                                    int it) {
+  for_each_item(w, [&](const SimParams& P, uint32_t t, uint32_t) {
+    body_match_body<kBodyBlockBatched, kBodyHeldBatched>(P, d, t, it);
+  });
 }
 
 // bodyDrag (src/wgsl.js:187-214) over the held body's particle list.
@@ -273,10 +308,12 @@ void launch_body_match(const SimParams& P, const DevScene& d, int it, cudaStream
   k_body_match<<<P.nBodies, kBodyBlock, 0, st>>>(P, d, it);
 }
 void launch_body_seed_b(const BatchWork& w, int maxItems, const DevScene& d, cudaStream_t st) {
-  k_body_seed_b<<<persistent_grid((const void*)k_body_seed_b, kBodyBlock, maxItems), kBodyBlock, 0, st>>>(w, d);
+  const int grid = persistent_grid((const void*)k_body_seed_b, kBodyBlockBatched, maxItems);
+  k_body_seed_b<<<grid, kBodyBlockBatched, 0, st>>>(w, d);
 }
 void launch_body_match_b(const BatchWork& w, int maxItems, const DevScene& d, int it, cudaStream_t st) {
-  k_body_match_b<<<persistent_grid((const void*)k_body_match_b, kBodyBlock, maxItems), kBodyBlock, 0, st>>>(w, d, it);
+  const int grid = persistent_grid((const void*)k_body_match_b, kBodyBlockBatched, maxItems);
+  k_body_match_b<<<grid, kBodyBlockBatched, 0, st>>>(w, d, it);
 }
 
 void launch_body_drag(const DevScene& d, float4* vel, const uint4* body, uint32_t held,
