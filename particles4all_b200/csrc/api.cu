@@ -50,6 +50,22 @@ const char* const kPhaseNames[PH_COUNT] = {
 std::atomic<uint64_t> g_launches{0};
 }  // namespace
 
+// A frame's launches as p4a_step captured them, and all that decides what they are: the
+// parameters (with the parity of the frame's first sort, substeps and iterations), the
+// buffers, and the launch shapes.
+struct FrameKey {
+  SimParams P;
+  DevScene d;
+  int32_t lanes, tension, bodies, shape[TK_COUNT];
+};
+struct FrameGraph {
+  FrameKey key;
+  cudaGraphExec_t exec = nullptr;
+  uint64_t launches = 0, used = 0;  // used: the sim's frame count when the key last came up
+  int seen = 0;                     // times it came up again without a graph
+};
+constexpr int kFrameGraphs = 4;
+
 struct p4a_sim {
   int device = 0;
   cudaStream_t stream = nullptr;
@@ -80,7 +96,10 @@ struct p4a_sim {
   int heldBody = -1;
   double heldTarget[3] = {0, 0, 0}, heldRate = 10, heldLimit = 4;
   SimParams P{};
-  uint32_t scanEpoch = 0;
+  FrameGraph frames[kFrameGraphs];  // p4a_step
+  uint64_t frameUse = 0;
+  cudaStream_t captureStream = nullptr;
+  uint64_t* captured = nullptr;  // while a frame is captured: where its launches are counted
   // readback (stats, error word, pose), latest-completed semantics
   uint32_t* pinned = nullptr;  // [8 stats][1 err][pad] then pose floats
   size_t pinnedBytes = 0;
@@ -205,9 +224,13 @@ int resolve_marks(p4a_sim* s) {
 
 // Called before each kernel the handle launches (and with PH_END after the last):
 // counts launches and, with profiling on, records the event that opens the interval.
+void note_launch(p4a_sim* s) {
+  if (s->captured) ++*s->captured;
+  else count_launches(1);
+}
 void mark(p4a_sim* s, int phase) {
   // the SSFR phase counts its own launches (several kernels per phase)
-  if (phase < PH_COUNT && phase != PH_STATS_CLEAR && phase != PH_SSFR && phase != PH_RAY) g_launches.fetch_add(1, std::memory_order_relaxed);
+  if (phase < PH_COUNT && phase != PH_STATS_CLEAR && phase != PH_SSFR && phase != PH_RAY) note_launch(s);
   if (!s->prof) return;
   if (s->evUsed == (int)s->evPool.size()) {
     cudaEvent_t e;
@@ -315,12 +338,6 @@ void pack_params(p4a_sim* s, double dt) {
 constexpr int kGroup16 = 6000, kGroup8 = 20000;
 int group_lanes(int n) { return n <= kGroup16 ? 16 : n <= kGroup8 ? 8 : 0; }
 
-uint32_t next_epoch(p4a_sim* s) {
-  s->scanEpoch = (s->scanEpoch + 1) & 0x3fffffffu;
-  if (s->scanEpoch == 0) s->scanEpoch = 1;
-  return s->scanEpoch;
-}
-
 // Cell arrays: histogram, cellStart, scan tile state (src/sim.js:107-110).
 int alloc_cells(p4a_sim* s) {
   free_list(s->cellAllocs);
@@ -365,8 +382,7 @@ void grid_pass(p4a_sim* s, int par) {
   mark(s, PH_KEY_COUNT);
   launch_key_count(s->P, d, st);
   mark(s, PH_SCAN);
-  launch_scan(d.cellCount, d.cellStart, s->nCells, d.scanState, d.scanTicket, next_epoch(s),
-              d.errorWord, st);
+  launch_scan(d.cellCount, d.cellStart, s->nCells, d.scanState, d.scanTicket, 0u, d.errorWord, st);
   mark(s, PH_FILL);
   launch_fill(s->P, d, st);
   mark(s, PH_REORDER);
@@ -518,6 +534,140 @@ int check_error_word(p4a_sim* s) {
   if (w & ERR_SCAN_TIMEOUT)
     return fail(s, P4A_ERR_TIMEOUT, "cell scan: a bounded wait on a predecessor tile gave up");
   return P4A_OK;
+}
+
+// The launches of a frame of `sub` substeps (src/sim.js:463-572), on the sim's stream.
+int enqueue_frame(p4a_sim* s, int sub) {
+  const p4a_params& p = s->params;
+  const SimParams& P = s->P;
+  const double dt = 1.0 / 60 / std::max(1, p.substeps);
+  DevScene& d = s->d;
+  cudaStream_t st = s->stream;
+  const bool bodies = s->nBodyParts > 0 && s->nBodies > 0;
+  const bool dragging = s->heldBody >= 1 && s->nBodyParts > 0;
+  const float blend = (float)(1 - std::exp(-std::max(dt, 0.0) / 0.02));
+  const float goal[3] = {(float)s->heldTarget[0], (float)s->heldTarget[1], (float)s->heldTarget[2]};
+  const int iters = std::max(1, p.iterations);
+  const bool tension = p.surface_tension_k > 0;
+  const int G = group_lanes(s->n);
+  for (int step = 0; step < sub; step++) {
+    const int par = s->parity, q = par ^ 1;
+    if (dragging) {
+      const uint32_t hb = (uint32_t)s->heldBody;
+      mark(s, PH_DRAG);
+      launch_body_drag(d, d.vel[par], d.body[par], hb, s->bodyStartHost[hb] - s->bodyStartHost[hb - 1],
+                       s->bodyStartHost[hb - 1], goal, (float)s->heldRate, blend, (float)s->heldLimit, st);
+    }
+    grid_pass(s, par);  // sets P.parity = par: the passes below read parity par ^ 1
+    s->parity = q;
+    s->predParity = q;
+    if (bodies) {
+      mark(s, PH_BODY_SEED);
+      launch_body_seed(P, d, st);
+    }
+    for (int it = 0; it < iters; it++) {
+      mark(s, PH_LAMBDA);
+      if (G) launch_lambda_g(P, d, it, G, st);
+      else launch_lambda(P, d, it, st);
+      mark(s, PH_DELTA);
+      if (G) launch_delta_g(P, d, it, G, st);
+      else launch_delta(P, d, it, st);
+      if (bodies) {
+        mark(s, PH_BODY_MATCH);
+        launch_body_match(P, d, it, st);
+      }
+    }
+    if (step == sub - 1) {
+      mark(s, PH_STATS_CLEAR);
+      CUDA_TRY(s, cudaMemsetAsync(d.statsOut, 0, 32, st));
+    }
+    if (tension) {
+      mark(s, PH_XSPH_NORMALS);
+      if (G) launch_xsph_normals_g(P, d, G, st);
+      else launch_xsph_normals(P, d, st);
+      mark(s, PH_TENSION_FINALIZE);
+      if (G) launch_tension_finalize_g(P, d, G, st);
+      else launch_tension_finalize(P, d, step, st);
+    } else {
+      mark(s, PH_XSPH_FINALIZE);
+      if (G) launch_xsph_finalize_g(P, d, G, st);
+      else launch_xsph_finalize(P, d, step, st);
+    }
+    if (G && step == sub - 1) {
+      note_launch(s);
+      launch_stats(P, d, st);
+    }
+  }
+  return P4A_OK;
+}
+
+// The graph of the coming frame (P packed, subs set), or null: the frame is enqueued
+// launch by launch. A launch costs the host about 3 us and leaves a gap of about a
+// microsecond on the device, which is most of a small scene's frame; a graph of the same
+// launches costs one. us a frame, three scenes side by side: 2,197 particles 90 -> 56,
+// 32,768 164 -> 145, the preset of 62,742 with bodies 898 -> 855, 263,872 with bodies
+// 812 -> 799. Capturing costs about 170 us once, so a frame becomes a graph when its key
+// has come up twice before: a scene whose parameters, particle count or buffers change
+// from frame to frame never pays for one.
+FrameGraph* frame_graph(p4a_sim* s, int sub) {
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  if (cudaStreamIsCapturing(s->stream, &cap) != cudaSuccess || cap != cudaStreamCaptureStatusNone) {
+    cudaGetLastError();
+    return nullptr;
+  }
+  FrameKey key;
+  memset(&key, 0, sizeof(key));
+  key.P = s->P;
+  key.P.parity = (uint32_t)s->parity;
+  key.d = s->d;
+  key.lanes = group_lanes(s->n);
+  key.tension = s->params.surface_tension_k > 0;
+  key.bodies = s->nBodyParts > 0 && s->nBodies > 0;
+  for (int k = 0; k < TK_COUNT; k++) key.shape[k] = tuned_variant(k, s->n);
+  s->frameUse++;
+  FrameGraph *f = nullptr, *oldest = s->frames;
+  for (FrameGraph& g : s->frames) {
+    if (g.used && memcmp(&g.key, &key, sizeof(key)) == 0) f = &g;
+    if (g.used < oldest->used) oldest = &g;
+  }
+  if (!f) {
+    if (oldest->exec) cudaGraphExecDestroy(oldest->exec);
+    *oldest = FrameGraph{};
+    memcpy(&oldest->key, &key, sizeof(key));
+    oldest->used = s->frameUse;
+    return nullptr;
+  }
+  f->used = s->frameUse;
+  if (f->exec || ++f->seen < 2) return f->exec ? f : nullptr;
+  // capture on a stream of the handle's own: the sim's may be one that cannot be captured
+  const int parity = s->parity, predParity = s->predParity;
+  const SimParams P = s->P;
+  cudaStream_t st = s->stream;
+  cudaGraph_t graph = nullptr;
+  bool ok = s->captureStream || cudaStreamCreateWithFlags(&s->captureStream, cudaStreamNonBlocking) == cudaSuccess;
+  if (ok && cudaStreamBeginCapture(s->captureStream, cudaStreamCaptureModeThreadLocal) == cudaSuccess) {
+    s->stream = s->captureStream;
+    f->launches = 0;
+    s->captured = &f->launches;
+    ok = enqueue_frame(s, sub) == P4A_OK;
+    s->captured = nullptr;
+    s->stream = st;
+    ok = cudaStreamEndCapture(s->captureStream, &graph) == cudaSuccess && ok;
+    ok = ok && cudaGraphInstantiate(&f->exec, graph, 0) == cudaSuccess;
+    if (graph) cudaGraphDestroy(graph);
+  } else {
+    ok = false;
+  }
+  s->parity = parity;
+  s->predParity = predParity;
+  s->P = P;
+  if (!ok) {
+    f->exec = nullptr;
+    f->seen = -(1 << 30);  // not tried again
+    cudaGetLastError();
+    return nullptr;
+  }
+  return f;
 }
 
 // Queues the copy of statsOut, the error word and the body pose into pinned memory
@@ -718,6 +868,9 @@ int p4a_destroy(p4a_sim* s) {
   if (s->raySurf) cudaFree(s->raySurf);
   if (s->rayRanges) cudaFree(s->rayRanges);
   if (s->envCube) cudaFree(s->envCube);
+  for (FrameGraph& f : s->frames)
+    if (f.exec) cudaGraphExecDestroy(f.exec);
+  if (s->captureStream) cudaStreamDestroy(s->captureStream);
   if (s->pinned) cudaFreeHost(s->pinned);
   if (s->readEvent) cudaEventDestroy(s->readEvent);
   for (cudaEvent_t e : s->evPool) cudaEventDestroy(e);
@@ -834,66 +987,21 @@ int p4a_step(p4a_sim* s, double frameDt, int32_t* substeps_out) {
     if (rc) return rc;
   }
   pack_params(s, dt);
-  const SimParams& P = s->P;
-  DevScene& d = s->d;
+  s->P.subs = (uint32_t)sub;
+  SimParams& P = s->P;
   cudaStream_t st = s->stream;
-  const bool bodies = s->nBodyParts > 0 && s->nBodies > 0;
   const bool dragging = s->heldBody >= 1 && s->nBodyParts > 0;
-  const float blend = (float)(1 - std::exp(-std::max(dt, 0.0) / 0.02));
-  const float goal[3] = {(float)s->heldTarget[0], (float)s->heldTarget[1], (float)s->heldTarget[2]};
-  const int iters = std::max(1, p.iterations);
-  const bool tension = p.surface_tension_k > 0;
-  const int G = group_lanes(s->n);
-  for (int step = 0; step < sub; step++) {
-    const int par = s->parity, q = par ^ 1;
-    if (dragging) {
-      const uint32_t hb = (uint32_t)s->heldBody;
-      mark(s, PH_DRAG);
-      launch_body_drag(d, d.vel[par], d.body[par], hb, s->bodyStartHost[hb] - s->bodyStartHost[hb - 1],
-                       s->bodyStartHost[hb - 1], goal, (float)s->heldRate, blend, (float)s->heldLimit, st);
-    }
-    s->P.subs = (uint32_t)sub;
-    grid_pass(s, par);  // sets P.parity = par: the passes below read parity par ^ 1
-    s->parity = q;
-    s->predParity = q;
-    if (bodies) {
-      mark(s, PH_BODY_SEED);
-      launch_body_seed(P, d, st);
-    }
-    for (int it = 0; it < iters; it++) {
-      mark(s, PH_LAMBDA);
-      if (G) launch_lambda_g(P, d, it, G, st);
-      else launch_lambda(P, d, it, st);
-      mark(s, PH_DELTA);
-      if (G) launch_delta_g(P, d, it, G, st);
-      else launch_delta(P, d, it, st);
-      if (bodies) {
-        mark(s, PH_BODY_MATCH);
-        launch_body_match(P, d, it, st);
-      }
-    }
-    if (step == sub - 1) {
-      mark(s, PH_STATS_CLEAR);
-      CUDA_TRY(s, cudaMemsetAsync(d.statsOut, 0, 32, st));
-    }
-    if (tension) {
-      mark(s, PH_XSPH_NORMALS);
-      if (G) launch_xsph_normals_g(P, d, G, st);
-      else launch_xsph_normals(P, d, st);
-      mark(s, PH_TENSION_FINALIZE);
-      if (G) launch_tension_finalize_g(P, d, G, st);
-      else launch_tension_finalize(P, d, step, st);
-    } else {
-      mark(s, PH_XSPH_FINALIZE);
-      if (G) launch_xsph_finalize_g(P, d, G, st);
-      else launch_xsph_finalize(P, d, step, st);
-    }
-    if (G && step == sub - 1) {
-      count_launches(1);
-      launch_stats(P, d, st);
-    }
-    s->simTime += dt;
+  FrameGraph* f = dragging || s->prof ? nullptr : frame_graph(s, sub);
+  if (f) {
+    CUDA_TRY(s, cudaGraphLaunch(f->exec, st));
+    count_launches(f->launches);
+    s->parity = s->predParity = s->parity ^ (sub & 1);
+    P.parity = (uint32_t)s->parity ^ 1u;
+  } else {
+    const int rc = enqueue_frame(s, sub);
+    if (rc) return rc;
   }
+  for (int step = 0; step < sub; step++) s->simTime += dt;
   if (sub > 0) s->sortedMoves = true;
   mark(s, PH_END);
   CUDA_TRY(s, cudaGetLastError());

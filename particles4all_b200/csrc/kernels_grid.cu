@@ -286,8 +286,17 @@ __global__ void __launch_bounds__(kBlock) k_scan(uint32_t* __restrict__ cellCoun
                                                  unsigned long long* __restrict__ state,
                                                  uint32_t* __restrict__ ticket, uint32_t epoch,
                                                  int nTiles, uint32_t* __restrict__ err, uint32_t spinLimit) {
-  __shared__ uint32_t s_tile;
-  if (threadIdx.x == 0) s_tile = atomicAdd(ticket, 1u);
+  __shared__ uint32_t s_tile, s_epoch;
+  if (threadIdx.x == 0) {
+    if (epoch != 0u) {
+      s_tile = atomicAdd(ticket, 1u);
+      s_epoch = epoch;
+    } else {  // the last scan's epoch is kept above the ticket: one atomic reads both
+      const unsigned long long w = atomicAdd(reinterpret_cast<unsigned long long*>(ticket), 1ull);
+      s_tile = (uint32_t)w;
+      s_epoch = (uint32_t)(w >> 32) >= 0x3fffffffu ? 1u : (uint32_t)(w >> 32) + 1u;
+    }
+  }
   __syncthreads();
   const int tile = (int)s_tile;
   if (tile >= nTiles) {  // only after an earlier launch failed mid-way: never index past the state
@@ -295,8 +304,11 @@ __global__ void __launch_bounds__(kBlock) k_scan(uint32_t* __restrict__ cellCoun
     return;
   }
   scan_tile(cellCount, cellStart, (long long)tile * kScanTile, nCells, tile, 0, 0u,
-            tile == nTiles - 1, state, epoch, err, spinLimit);
-  if (threadIdx.x == 0 && tile == nTiles - 1) *ticket = 0u;  // all tickets taken: reset
+            tile == nTiles - 1, state, s_epoch, err, spinLimit);
+  if (threadIdx.x == 0 && tile == nTiles - 1) {  // all tickets taken: reset
+    if (epoch != 0u) *ticket = 0u;
+    else *reinterpret_cast<unsigned long long*>(ticket) = (unsigned long long)s_epoch << 32;
+  }
 }
 
 // Batched: a three-phase scan with no waiting, over items[g] = (scene slot, local

@@ -309,6 +309,8 @@ inline int scan_tiles(int nCells) { return groups(nCells, kScanTile); }
 
 // ---- plain launchers (one scene; P.parity = live parity before the sort) ----
 void launch_key_count(const SimParams& P, const DevScene& d, cudaStream_t st);
+// `epoch` tags the tile states of this scan, other than the last one's; 0: counted on the
+// device in the upper half of the 8-byte aligned word at `ticket` (a replayed launch).
 void launch_scan(uint32_t* cellCount, uint32_t* cellStart, int nCells,
                  unsigned long long* state, uint32_t* ticket, uint32_t epoch, uint32_t* err,
                  cudaStream_t st, uint32_t spinLimit = kScanSpinLimit);
