@@ -360,7 +360,7 @@ int upload_boundary(p4a_sim* s) {
   const int nb = hb.count;
   if ((rc = dalloc(s, s->boundaryAllocs, &s->d.bpos, (size_t)std::max(1, nb)))) return rc;
   if ((rc = dalloc(s, s->boundaryAllocs, &s->d.bpsi, (size_t)std::max(1, nb)))) return rc;
-  if ((rc = dalloc(s, s->boundaryAllocs, &s->d.bsample, (size_t)std::max(1, nb)))) return rc;
+  if ((rc = dalloc(s, s->boundaryAllocs, &s->d.bsample, (size_t)nb + kReadPad))) return rc;
   if ((rc = dalloc(s, s->boundaryAllocs, &s->d.bcellStart, (size_t)s->nCells + 2))) return rc;
   std::vector<float> sample(hb.pos);
   for (int k = 0; k < nb; k++) sample[(size_t)k * 4 + 3] = hb.psi[k];
@@ -411,7 +411,7 @@ int reset_common(p4a_sim* s) {
   auto& L = s->sceneAllocs;
   for (int t = 0; t < 2; t++) {
     if ((rc = dalloc(s, L, &s->d.pos[t], cap)) || (rc = dalloc(s, L, &s->d.vel[t], cap)) ||
-        (rc = dalloc(s, L, &s->d.pred[t], cap)) || (rc = dalloc(s, L, &s->d.body[t], cap)) ||
+        (rc = dalloc(s, L, &s->d.pred[t], cap + kReadPad)) || (rc = dalloc(s, L, &s->d.body[t], cap)) ||
         (rc = dalloc(s, L, &s->d.rest[t], cap)))
       return rc;
   }

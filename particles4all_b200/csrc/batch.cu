@@ -843,7 +843,7 @@ int alloc_arenas(p4a_batch* b) {
   DevScene& d = b->d;
   int rc = P4A_OK;
   for (int t = 0; t < 2 && !rc; t++) {
-    if ((rc = balloc(b, &d.pos[t], P)) || (rc = balloc(b, &d.vel[t], P)) || (rc = balloc(b, &d.pred[t], P)) ||
+    if ((rc = balloc(b, &d.pos[t], P)) || (rc = balloc(b, &d.vel[t], P)) || (rc = balloc(b, &d.pred[t], P + kReadPad)) ||
         (rc = balloc(b, &d.body[t], P)) || (rc = balloc(b, &d.rest[t], P)))
       break;
   }
@@ -858,7 +858,7 @@ int alloc_arenas(p4a_batch* b) {
        (rc = balloc(b, &d.cellCount, Cc)) ||
        (rc = balloc(b, &d.cellStart, Cc)) || (rc = balloc(b, &d.bcellStart, Cc)) ||
        (rc = balloc(b, &d.scanState, b->scanTilesCap)) || (rc = balloc(b, &d.scanTicket, 4)) ||
-       (rc = balloc(b, &d.errorWord, 4)) || (rc = balloc(b, &d.bsample, b->cfg.max_boundary)) ||
+       (rc = balloc(b, &d.errorWord, 4)) || (rc = balloc(b, &d.bsample, b->cfg.max_boundary + kReadPad)) ||
        (rc = balloc(b, &d.bodyAccum, B1 * 4)) ||
        (rc = balloc(b, &d.bodyCov, B1 * 9)) || (rc = balloc(b, &d.bodyCentre, B1)) ||
        (rc = balloc(b, &d.bodyRef, B1)) || (rc = balloc(b, &d.bodyRot, B1 * 3)) ||

@@ -58,11 +58,36 @@ struct RowWalk {
   }
 };
 
+// Bit k: point k of pts[0, n), n <= 32, lies within r^2 < r2lim of p. Reads whole groups
+// of four points: position arrays have kReadPad elements more than they hold particles.
+__device__ __forceinline__ uint32_t near_bits(F3 p, const float4* __restrict__ pts, uint32_t n, float r2lim) {
+  uint32_t m = 0u;
+#pragma unroll 1
+  for (uint32_t k = 0; k < n; k += 4u) {
+    const float4 q0 = __ldg(&pts[k]), q1 = __ldg(&pts[k + 1]), q2 = __ldg(&pts[k + 2]), q3 = __ldg(&pts[k + 3]);
+    const F3 d0 = sub3(p, xyz(q0)), d1 = sub3(p, xyz(q1)), d2 = sub3(p, xyz(q2)), d3 = sub3(p, xyz(q3));
+    uint32_t g = dot3(d0, d0) < r2lim ? 1u : 0u;
+    if (dot3(d1, d1) < r2lim) g |= 2u;
+    if (dot3(d2, d2) < r2lim) g |= 4u;
+    if (dot3(d3, d3) < r2lim) g |= 8u;
+    m |= g << k;
+  }
+  return m & (0xffffffffu >> (32u - n));
+}
+
 // Phase 1: the list of particle i (scene-local cellStart cs / bcs, arena index i)
 // with every candidate j != i of the nine rows within r^2 < r2lim, and, when B,
 // every boundary sample of each row within r^2 < r2lim after the row's fluid
 // candidates. Returns the entry count (| kHasBound when boundary samples were
 // listed), or kListOverflow.
+// A row's candidates are tested first, into a bit mask, and only the ones within the
+// radius are then appended: of the 27 cells' 216 candidates about 35 are, and some lane of
+// a warp has one at nearly every candidate, so appending as they are tested runs the
+// append 216 times. What is left is bound by the loads of the candidates: 16 bytes for
+// each lane, four cycles of the L1 each (88 % busy). us per launch of lambda, a list built
+// in every launch (preset, 62,742) 68.9 -> 48.2, in the first of a substep's (one scene of
+// 32,768 / 264k / 2.1M) 28.1 -> 26.3 / 56.4 -> 55.5 / 284 -> 276, 96 mixed scenes
+// 539 -> 492; xsph with a list of its own (preset) 74.5 -> 59.7.
 template <bool B>
 __device__ __forceinline__ uint32_t build_list(const SimParams& P, const RowWalk& w, uint32_t i, F3 pi,
                                                const float4* __restrict__ pred,
@@ -73,48 +98,36 @@ __device__ __forceinline__ uint32_t build_list(const SimParams& P, const RowWalk
   uint32_t c = 0, flags = 0u, held = 0u;
   // entries are stored two at a time: `held` is the first of a pair
   uint2* __restrict__ out = reinterpret_cast<uint2*>(list) + i;
-  auto push = [&](uint32_t e) {
-    if ((c & 1u) != 0u && c < kListCap) {
-      *out = make_uint2(held, e);
-      out += cap;
+  // appends the points of [b, e) within the radius, 32 candidates at a time
+  auto row = [&](const float4* __restrict__ pts, uint32_t b, uint32_t e, uint32_t tag) {
+#pragma unroll 1
+    for (uint32_t base = b; base < e; base += 32u) {
+      const uint32_t n = min(e - base, 32u);
+      uint32_t m = near_bits(pi, pts + base, n, r2lim);
+      if (tag == 0u && i - base < 32u) m &= ~(1u << (i - base));
+      if (c + (uint32_t)__popc(m) > kListCap) {  // overflow: the list is not used
+        c = kListCap + 1u;
+        m = 0u;
+      }
+      if (tag != 0u && m != 0u) flags = kHasBound;
+      for (; m != 0u; m &= m - 1u) {
+        const uint32_t at = tag | (base + (uint32_t)__ffs((int)m) - 1u);
+        if ((c & 1u) != 0u) {
+          *out = make_uint2(held, at);
+          out += cap;
+        }
+        held = at;
+        c++;
+      }
     }
-    held = e;
-    c++;
   };
 #pragma unroll 1
   for (int r = 0; r < kRows; r++) {
     const int rb = w.row_base(P, r);
     if (rb < 0) continue;
-    const uint32_t b = __ldg(&cs[rb + w.x0]);
-    const uint32_t e = min(__ldg(&cs[rb + w.x1 + 1]), P.pEnd);
-    uint32_t j = b;
-    for (; j + 4 <= e; j += 4) {
-      const float4 q0 = __ldg(&pred[j]), q1 = __ldg(&pred[j + 1]);
-      const float4 q2 = __ldg(&pred[j + 2]), q3 = __ldg(&pred[j + 3]);
-      const F3 d0 = sub3(pi, xyz(q0)), d1 = sub3(pi, xyz(q1));
-      const F3 d2 = sub3(pi, xyz(q2)), d3 = sub3(pi, xyz(q3));
-      const bool i0 = dot3(d0, d0) < r2lim, i1 = dot3(d1, d1) < r2lim;
-      const bool i2 = dot3(d2, d2) < r2lim, i3 = dot3(d3, d3) < r2lim;
-      if (i0 && j != i) push(j);
-      if (i1 && j + 1 != i) push(j + 1);
-      if (i2 && j + 2 != i) push(j + 2);
-      if (i3 && j + 3 != i) push(j + 3);
-    }
-    for (; j < e; j++) {
-      const F3 d0 = sub3(pi, xyz(__ldg(&pred[j])));
-      if (dot3(d0, d0) < r2lim && j != i) push(j);
-    }
+    row(pred, __ldg(&cs[rb + w.x0]), min(__ldg(&cs[rb + w.x1 + 1]), P.pEnd), 0u);
     if constexpr (B) {
-      if (P.nBoundary > 0u) {
-        const uint32_t bb = __ldg(&bcs[rb + w.x0]), be = __ldg(&bcs[rb + w.x1 + 1]);
-        for (uint32_t k = bb; k < be; k++) {
-          const F3 d0 = sub3(pi, xyz(__ldg(&bpos[k])));
-          if (dot3(d0, d0) < r2lim) {
-            push(kBoundTag | k);
-            flags = kHasBound;
-          }
-        }
-      }
+      if (P.nBoundary > 0u) row(bpos, __ldg(&bcs[rb + w.x0]), __ldg(&bcs[rb + w.x1 + 1]), kBoundTag);
     }
   }
   if ((c & 1u) != 0u && c < kListCap) *out = make_uint2(held, i);
@@ -183,7 +196,7 @@ __device__ __forceinline__ uint32_t build_list_coop(const SimParams& P, const Ro
 // (build_list_coop), instead of letting the warp wait while those lanes test
 // their ~216 candidates one by one; when many do, each lane builds its own.
 // Returns the lane's new count word, or `current` for lanes that need none.
-constexpr int kCoopLanes = 12;
+constexpr int kCoopLanes = 2;
 template <bool B>
 __device__ __forceinline__ uint32_t build_lists_warp(const SimParams& P, bool need, const RowWalk& w, uint32_t i,
                                                      F3 pi, const float4* __restrict__ pred,

@@ -230,6 +230,9 @@ enum : uint32_t { ERR_SCAN_TIMEOUT = 1u, ERR_BODY_OVERFLOW = 2u };
 // Device buffers of a scene, or of the arenas of a batch (same layout).
 constexpr uint32_t kListCap = 96;  // neighbour-list entries per particle (nbList)
 
+// Elements that pred and bsample are longer than what they hold (near_bits reads whole
+// groups of four).
+constexpr size_t kReadPad = 4;
 struct DevScene {
   float4* pos[2];
   float4* vel[2];
