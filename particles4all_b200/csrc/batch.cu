@@ -146,6 +146,7 @@ struct Frame {
   std::vector<SimParams> params;
   int nSubs = 0, nRows = 0;
   int variant[TK_COUNT] = {0, 0, 0, 0};  // launch shapes of the tuned kernels
+  bool far = false;                      // far_lists of the frame's particles
   std::vector<int> shape;
 };
 
@@ -201,7 +202,7 @@ int run_frame(p4a_batch* b, const Frame& F, bool graphForm, uint64_t* launched,
       case LK_REORDER: launch_reorder_b(w, maxItems, d, st); break;
       case LK_SEED: launch_body_seed_b(w, maxItems, d, st); break;
       case LK_LAMBDA: launch_lambda_b(w, maxItems, d, r.it, st, F.variant[TK_LAMBDA]); break;
-      case LK_DELTA: launch_delta_b(w, maxItems, d, r.it, st, F.variant[TK_DELTA]); break;
+      case LK_DELTA: launch_delta_b(w, maxItems, d, r.it, F.far, st, F.variant[TK_DELTA]); break;
       case LK_MATCH: launch_body_match_b(w, maxItems, d, r.it, st); break;
       case LK_FINISH: launch_xsph_finalize_b(w, maxItems, d, r.sub, st); break;
       case LK_NORMALS: launch_xsph_normals_b(w, maxItems, d, st, F.variant[TK_NORMALS]); break;
@@ -667,6 +668,8 @@ int step_frame(p4a_batch* b, const int32_t* ids, const double* frameDt, int32_t 
     F.variant[k] = tuned_variant_batched(k, total);
     F.shape.push_back(F.variant[k]);
   }
+  F.far = far_lists(total);
+  F.shape.push_back(F.far);
   F.shape.push_back(maxSub);
   WorkSeg zero{0, 0};
   for (int k = 0; k < count; k++)

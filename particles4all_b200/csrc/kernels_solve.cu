@@ -37,13 +37,13 @@ namespace p4a {
 // takes 525 us per launch on the 96-scene mix in halves (728 us one entry at a time with
 // the IEEE operations), delta 327 us (426 us); on the large scene 269 us (289 us) and
 // 178 us (232 us).
-template <bool B>
+template <bool B, bool FAR>
 __device__ __forceinline__ void lambda_walk(const SimParams& P, const DevScene& d, uint32_t i, uint32_t count, F3 pi,
                                             const float4* __restrict__ pred, float& rho, F3& gradSum,
                                             float& sumGrad2) {
   const F2 one = splat2(-1.0f), h2 = splat2(P.h2), h = splat2(P.h), poly = splat2(P.poly6);
   const F2 cFluid = splat2(-P.volSpiky);
-  walk2<B>(d.nbList, d.cap, i, count, pred, d.bsample, [&](uint2 e, float4 q0, float4 q1) {
+  walk2<B, FAR>(d.nbList, d.cap, i, count, pred, d.bsample, [&](uint2 e, float4 q0, float4 q1) {
     const F3 r0 = sub3(pi, xyz(q0)), r1 = sub3(pi, xyz(q1));
     const float x0 = dot3(r0, r0), x1 = dot3(r1, r1);
     const bool b0 = B && (e.x & kBoundTag) != 0u, b1 = B && (e.y & kBoundTag) != 0u;
@@ -81,6 +81,7 @@ __device__ __forceinline__ void lambda_walk(const SimParams& P, const DevScene& 
 
 // Called by all 32 lanes of a warp (lanes past the scene's end only take part in the
 // warp's list builds).
+template <bool FAR>
 __device__ __forceinline__ void lambda_body(const SimParams& P, const DevScene& d, uint32_t li, int it) {
   const bool act = li < P.n;
   const uint32_t i = P.pOff + (act ? li : 0u);
@@ -109,9 +110,9 @@ __device__ __forceinline__ void lambda_body(const SimParams& P, const DevScene& 
   if (count != kListOverflow && (P.pairMath & PAIR_SOLVE) != 0u) {
     // warps without a boundary sample in any list skip the kind selects
     if (__any_sync(__activemask(), (count & kHasBound) != 0u)) {
-      lambda_walk<true>(P, d, i, count, pi, pred, rho, gradSum, sumGrad2);
+      lambda_walk<true, FAR>(P, d, i, count, pi, pred, rho, gradSum, sumGrad2);
     } else {
-      lambda_walk<false>(P, d, i, count, pi, pred, rho, gradSum, sumGrad2);
+      lambda_walk<false, FAR>(P, d, i, count, pi, pred, rho, gradSum, sumGrad2);
     }
   } else {
     auto fluid = [&](uint32_t, float4 q) {
@@ -164,13 +165,13 @@ __device__ __forceinline__ void lambda_body(const SimParams& P, const DevScene& 
 
 // One list walk of delta, two entries at a time (B as in lambda_walk); nc counts the
 // fluid neighbours for sorAverage.
-template <bool B>
+template <bool B, bool FAR>
 __device__ __forceinline__ void delta_walk(const SimParams& P, const DevScene& d, uint32_t i, uint32_t count,
                                            float4 self, F3& dsum, F3& dB, float& nc) {
   const F2 one = splat2(-1.0f), h2 = splat2(P.h2), h = splat2(P.h), poly = splat2(P.poly6);
   const F2 cGrad = splat2(-P.spikyGrad), wq = splat2(P.sCorrWq), kc = splat2(-P.sCorrK);
   const F3 pi = xyz(self);
-  walk2<B>(d.nbList, d.cap, i, count, d.predLam, d.bsample, [&](uint2 e, float4 q0, float4 q1) {
+  walk2<B, FAR>(d.nbList, d.cap, i, count, d.predLam, d.bsample, [&](uint2 e, float4 q0, float4 q1) {
     const F3 r0 = sub3(pi, xyz(q0)), r1 = sub3(pi, xyz(q1));
     const float x0 = dot3(r0, r0), x1 = dot3(r1, r1);
     const bool in0 = !(x0 >= P.h2 || x0 < 1.0e-12f), in1 = !(x1 >= P.h2 || x1 < 1.0e-12f);
@@ -213,6 +214,7 @@ __device__ __forceinline__ void delta_walk(const SimParams& P, const DevScene& d
   });
 }
 
+template <bool FAR>
 __device__ __forceinline__ void delta_body(const SimParams& P, const DevScene& d, uint32_t li, int it) {
   if (li >= P.n) return;
   const uint32_t i = P.pOff + li;
@@ -226,9 +228,9 @@ __device__ __forceinline__ void delta_body(const SimParams& P, const DevScene& d
   float nc = 1.0f;
   if (count != kListOverflow && (P.pairMath & PAIR_SOLVE) != 0u) {
     if (__any_sync(__activemask(), (count & kHasBound) != 0u)) {
-      delta_walk<true>(P, d, i, count, self, dsum, dB, nc);
+      delta_walk<true, FAR>(P, d, i, count, self, dsum, dB, nc);
     } else {
-      delta_walk<false>(P, d, i, count, self, dsum, dB, nc);
+      delta_walk<false, FAR>(P, d, i, count, self, dsum, dB, nc);
     }
   } else {
     const float li_ = self.w;
@@ -271,36 +273,39 @@ __device__ __forceinline__ void delta_body(const SimParams& P, const DevScene& d
 
 // Plain: block b handles particles [b * TB, (b + 1) * TB). Batched: warps pull
 // 32-particle slices of the segment's tiles.
-template <int TB, int MB>
+template <int TB, int MB, bool FAR>
 __global__ void __launch_bounds__(TB, MB) k_lambda(const __grid_constant__ SimParams P,
                                                    const __grid_constant__ DevScene d, int it) {
-  lambda_body(P, d, blockIdx.x * TB + threadIdx.x, it);
+  lambda_body<FAR>(P, d, blockIdx.x * TB + threadIdx.x, it);
 }
 template <int TB, int MB>
 __global__ void __launch_bounds__(TB, MB) k_lambda_b(const __grid_constant__ BatchWork w,
                                                      const __grid_constant__ DevScene d, int it) {
-  for_each_slice(w, [&](const SimParams& P, uint32_t li) { lambda_body(P, d, li, it); });
+  for_each_slice(w, [&](const SimParams& P, uint32_t li) { lambda_body<false>(P, d, li, it); });
 }
 template <int TB, int MB>
 __global__ void __launch_bounds__(TB, MB) k_delta(const __grid_constant__ SimParams P,
                                                   const __grid_constant__ DevScene d, int it) {
-  delta_body(P, d, blockIdx.x * TB + threadIdx.x, it);
+  delta_body<false>(P, d, blockIdx.x * TB + threadIdx.x, it);
 }
-template <int TB, int MB>
+template <int TB, int MB, bool FAR>
 __global__ void __launch_bounds__(TB, MB) k_delta_b(const __grid_constant__ BatchWork w,
                                                     const __grid_constant__ DevScene d, int it) {
-  for_each_slice(w, [&](const SimParams& P, uint32_t li) { delta_body(P, d, li, it); });
+  for_each_slice(w, [&](const SimParams& P, uint32_t li) { delta_body<FAR>(P, d, li, it); });
 }
 
 using PlainFn = void (*)(SimParams, DevScene, int);
 using BatchFn = void (*)(BatchWork, DevScene, int);
-#define P4A_SHAPES(K, suffix)                                                                     \
-  {K##suffix<256, 4>, K##suffix<256, 3>, K##suffix<256, 5>, K##suffix<128, 8>, K##suffix<128, 6>, \
-   K##suffix<128, 10>}
-static const PlainFn kLambdaP[kVariants] = P4A_SHAPES(k_lambda, );
-static const BatchFn kLambdaB[kVariants] = P4A_SHAPES(k_lambda, _b);
-static const PlainFn kDeltaP[kVariants] = P4A_SHAPES(k_delta, );
-static const BatchFn kDeltaB[kVariants] = P4A_SHAPES(k_delta, _b);
+#define P4A_SHAPES(K, ...)                                                                           \
+  {K<256, 4 __VA_ARGS__>, K<256, 3 __VA_ARGS__>, K<256, 5 __VA_ARGS__>, K<128, 8 __VA_ARGS__>,       \
+   K<128, 6 __VA_ARGS__>, K<128, 10 __VA_ARGS__>}
+#define P4A_FAR(x) , x
+static const PlainFn kLambdaP[2][kVariants] = {P4A_SHAPES(k_lambda, P4A_FAR(false)),
+                                               P4A_SHAPES(k_lambda, P4A_FAR(true))};
+static const BatchFn kLambdaB[kVariants] = P4A_SHAPES(k_lambda_b);
+static const PlainFn kDeltaP[kVariants] = P4A_SHAPES(k_delta);
+static const BatchFn kDeltaB[2][kVariants] = {P4A_SHAPES(k_delta_b, P4A_FAR(false)),
+                                              P4A_SHAPES(k_delta_b, P4A_FAR(true))};
 
 static int pick(int kernel, int variant, int64_t n) {
   return variant >= 0 && variant < kVariants ? variant : tuned_variant(kernel, n);
@@ -308,7 +313,7 @@ static int pick(int kernel, int variant, int64_t n) {
 
 void launch_lambda(const SimParams& P, const DevScene& d, int it, cudaStream_t st, int variant) {
   const int v = pick(TK_LAMBDA, variant, P.n), tb = kShapes[TK_LAMBDA][v].threads;
-  kLambdaP[v]<<<groups(P.n, tb), tb, 0, st>>>(P, d, it);
+  kLambdaP[far_lists(P.n)][v]<<<groups(P.n, tb), tb, 0, st>>>(P, d, it);
 }
 void launch_delta(const SimParams& P, const DevScene& d, int it, cudaStream_t st, int variant) {
   const int v = pick(TK_DELTA, variant, P.n), tb = kShapes[TK_DELTA][v].threads;
@@ -318,9 +323,11 @@ void launch_lambda_b(const BatchWork& w, int maxItems, const DevScene& d, int it
   const int v = pick(TK_LAMBDA, variant, (int64_t)maxItems * kBlock), tb = kShapes[TK_LAMBDA][v].threads;
   kLambdaB[v]<<<persistent_grid((const void*)kLambdaB[v], tb, maxItems), tb, 0, st>>>(w, d, it);
 }
-void launch_delta_b(const BatchWork& w, int maxItems, const DevScene& d, int it, cudaStream_t st, int variant) {
+void launch_delta_b(const BatchWork& w, int maxItems, const DevScene& d, int it, bool far, cudaStream_t st,
+                    int variant) {
   const int v = pick(TK_DELTA, variant, (int64_t)maxItems * kBlock), tb = kShapes[TK_DELTA][v].threads;
-  kDeltaB[v]<<<persistent_grid((const void*)kDeltaB[v], tb, maxItems), tb, 0, st>>>(w, d, it);
+  const BatchFn k = kDeltaB[far][v];
+  k<<<persistent_grid((const void*)k, tb, maxItems), tb, 0, st>>>(w, d, it);
 }
 
 }  // namespace p4a

@@ -287,7 +287,8 @@ __device__ __forceinline__ bool list_reusable(const SimParams& P, const DevScene
 // pipelined: while a pair is processed, the next pair's gathers and the list load after
 // it are in flight, so the latency of the dependent list-then-gather chain overlaps
 // the arithmetic.
-template <bool B, class FPair>
+// With FAR the pair four ahead is prefetched into the L2: see far_lists.
+template <bool B, bool FAR, class FPair>
 __device__ __forceinline__ void walk2(const uint32_t* list, uint32_t cap, uint32_t i, uint32_t count,
                                       const float4* __restrict__ fsrc, const float4* __restrict__ bsrc,
                                       FPair&& pair) {
@@ -315,6 +316,7 @@ __device__ __forceinline__ void walk2(const uint32_t* list, uint32_t cap, uint32
       if (k + 1u < pairs) {
         at += cap;
         en = *at;
+        if (FAR && k + 4u < pairs) asm volatile("prefetch.global.L2 [%0];" ::"l"(at + 3 * (size_t)cap));
       }
     }
     pair(ec, c0, c1);

@@ -310,6 +310,15 @@ inline int groups(long long n, int per = kBlock) {
 }
 inline int scan_tiles(int nCells) { return groups(nCells, kScanTile); }
 
+// Whether the neighbour lists of n particles (about 140 bytes each are read in a pass) come
+// from DRAM in every pass rather than from the 126 MB L2, so that the walk of lambda (one
+// scene) and of delta (batched) prefetches them. us per launch without / with prefetch:
+// lambda 262,144 particles 53.4 / 55.8, 512,000 97.8 / 95.7, 729,000 130.7 / 126.1, 2.1M
+// with bodies 276 / 260; batched delta, 16 scenes of 1.5M in all 142 / 129, 96 scenes of 4M
+// 329 / 298. The other walks gain nothing from it (delta of one scene 182 / 182, batched
+// lambda 493 / 502, xsph+normals 323 / 338).
+inline bool far_lists(int64_t n) { return n >= 600000; }
+
 // ---- plain launchers (one scene; P.parity = live parity before the sort) ----
 void launch_key_count(const SimParams& P, const DevScene& d, cudaStream_t st);
 // `epoch` tags the tile states of this scan, other than the last one's; 0: counted on the
@@ -365,7 +374,8 @@ void launch_scan_apply_b(const BatchWork& w, int maxItems, const DevScene& d, cu
 void launch_fill_b(const BatchWork& w, int maxItems, const DevScene& d, cudaStream_t st);
 void launch_reorder_b(const BatchWork& w, int maxItems, const DevScene& d, cudaStream_t st);
 void launch_lambda_b(const BatchWork& w, int maxItems, const DevScene& d, int it, cudaStream_t st, int variant);
-void launch_delta_b(const BatchWork& w, int maxItems, const DevScene& d, int it, cudaStream_t st, int variant);
+void launch_delta_b(const BatchWork& w, int maxItems, const DevScene& d, int it, bool far, cudaStream_t st,
+                    int variant);
 void launch_body_seed_b(const BatchWork& w, int maxItems, const DevScene& d, cudaStream_t st);
 void launch_body_match_b(const BatchWork& w, int maxItems, const DevScene& d, int it, cudaStream_t st);
 void launch_xsph_finalize_b(const BatchWork& w, int maxItems, const DevScene& d, int substep, cudaStream_t st);

@@ -5,7 +5,7 @@ particle at every size; bit for bit the oracle."""
 import numpy as np
 import pytest
 
-from particles4all_b200 import Batch, configs
+from particles4all_b200 import Batch, Sim, configs
 from test_gpu_batch import assert_same
 from test_gpu_parity import compare, pair
 
@@ -42,3 +42,21 @@ def test_one_thread_per_particle_at_the_end_of_the_arrays(n):
         assert g.step(1 / 60) == o.step(1 / 60)
     compare(g, o)
     g.close()
+
+
+@pytest.mark.parametrize("side", [84, 85])
+def test_both_sides_of_the_prefetched_lists(side):
+    # 592,704 and 614,125 particles: in the batch lambda, alone delta never prefetches
+    p, sc = configs.dam_break_32k(side=side)
+    p = dict(p, box=[1.5 * side, side, side])
+    g = Sim()
+    g.reset_scene(p, sc)
+    b = Batch(max_particles=side ** 3, max_cells=1 << 23)
+    sid = b.add_scene(p, sc)
+    for _ in range(2):
+        g.step(1 / 60)
+        b.step([sid], 1 / 60)
+    assert_same(g, b, sid)
+    g.close()
+    b.close()
+
