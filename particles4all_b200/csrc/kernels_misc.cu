@@ -9,6 +9,7 @@
 
 #include "p4a_internal.h"
 #include "p4a_math.cuh"
+#include "pair_math.cuh"
 
 namespace p4a {
 
@@ -65,6 +66,13 @@ __device__ __forceinline__ float open_gap(int k, int n, float r, float support) 
   return fmaxf(fmaxf(below, above), 0.0f);
 }
 
+// One thread per particle over the candidates of up to 25 rows, bound by the instructions
+// issued (75 % of the slots) with 18 of 32 lanes in range at a candidate: FAST takes the
+// root of pair_math.cuh, which has no range test (5 instructions), and a row's last one to
+// three candidates are loaded together. 263,872 particles 357 -> 322 us. Testing a row
+// into a bit mask first, as the list builds do, took 340 us, a queue of the candidates in
+// range 390: the candidates in range are too many for the second visit to pay.
+template <bool FAST>
 __device__ __forceinline__ void aniso_body(const AnisoParams& A, const float4* __restrict__ pos,
                                            const uint32_t* __restrict__ cs, float4* __restrict__ smoothPos,
                                            float4* __restrict__ g, uint32_t i) {
@@ -124,7 +132,8 @@ __device__ __forceinline__ void aniso_body(const AnisoParams& A, const float4* _
         const F3 d = sub3(xyz(q), xi);
         const float r2 = dot3(d, d);
         if (r2 >= r2max) return;
-        const float t = sqrtf(r2) * invR;
+        // below 2^-96 the weight is 1 whatever the root
+        const float t = (FAST ? root1(r2 < 0x1p-96f ? 0x1p-96f : r2).s : sqrtf(r2)) * invR;
         const float w = 1.0f - t * t * t;
         sd = fma3(w, d, sd);
         m2.c[0] = fma3(d.x * w, d, m2.c[0]);
@@ -142,7 +151,12 @@ __device__ __forceinline__ void aniso_body(const AnisoParams& A, const float4* _
         cand(q2);
         cand(q3);
       }
-      for (; j < je; j++) cand(__ldg(&pos[j]));
+      if (j < je) {
+        const float4 q0 = __ldg(&pos[j]), q1 = __ldg(&pos[min(j + 1, je - 1)]), q2 = __ldg(&pos[min(j + 2, je - 1)]);
+        cand(q0);
+        if (j + 1 < je) cand(q1);
+        if (j + 2 < je) cand(q2);
+      }
     }
   }
   if (wsum <= 0.0f) {
@@ -221,22 +235,27 @@ void launch_resize(uint32_t n, float4* pos, const float oldSize[3], const float 
                                          F3{clampMax[0], clampMax[1], clampMax[2]});
 }
 
-template <int TB, int MB>
+template <int TB, int MB, bool FAST>
 __global__ void __launch_bounds__(TB, MB) k_aniso(const __grid_constant__ AnisoParams A,
                                                   const float4* __restrict__ pos,
                                                   const uint32_t* __restrict__ cs,
                                                   float4* __restrict__ smoothPos, float4* __restrict__ g) {
-  aniso_body(A, pos, cs, smoothPos, g, blockIdx.x * TB + threadIdx.x);
+  aniso_body<FAST>(A, pos, cs, smoothPos, g, blockIdx.x * TB + threadIdx.x);
 }
 using AnisoFn = void (*)(AnisoParams, const float4*, const uint32_t*, float4*, float4*);
-static const AnisoFn kAniso[kVariants] = {k_aniso<128, 10>, k_aniso<128, 8>, k_aniso<128, 12>,
-                                          k_aniso<256, 5>,  k_aniso<256, 4>, k_aniso<64, 20>};
+#define P4A_ANISO_SHAPES(F)                                                          \
+  {k_aniso<128, 10, F>, k_aniso<128, 8, F>, k_aniso<128, 12, F>, k_aniso<256, 5, F>, \
+   k_aniso<256, 4, F>, k_aniso<64, 20, F>}
+static const AnisoFn kAniso[2][kVariants] = {P4A_ANISO_SHAPES(false), P4A_ANISO_SHAPES(true)};
 
 void launch_aniso(const AnisoParams& A, const float4* pos, const uint32_t* cellStart,
                   float4* smoothPos, float4* g, cudaStream_t st, int variant) {
   const int v = variant >= 0 && variant < kVariants ? variant : tuned_variant(TK_ANISO, A.count);
   const int tb = kShapes[TK_ANISO][v].threads;
-  kAniso[v]<<<groups(A.count, tb), tb, 0, st>>>(A, pos, cellStart, smoothPos, g);
+  // r^2 stays within 2^-96 and 1e30, where the root is exact, and a weight at 2^-48 of the
+  // radius or less rounds to 1
+  const bool fast = A.radius >= 1.0e-10f && A.radius <= 1.0e15f;
+  kAniso[fast][v]<<<groups(A.count, tb), tb, 0, st>>>(A, pos, cellStart, smoothPos, g);
 }
 
 }  // namespace p4a

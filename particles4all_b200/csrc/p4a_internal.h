@@ -314,7 +314,7 @@ inline int scan_tiles(int nCells) { return groups(nCells, kScanTile); }
 // from DRAM in every pass rather than from the 126 MB L2, so that the walk of lambda (one
 // scene) and of delta (batched) prefetches them. us per launch without / with prefetch:
 // lambda 262,144 particles 53.4 / 55.8, 512,000 97.8 / 95.7, 729,000 130.7 / 126.1, 2.1M
-// with bodies 276 / 260; batched delta, 16 scenes of 1.5M in all 142 / 129, 96 scenes of 4M
+// with bodies 276 / 260; batched delta, 16 scenes of 1.1M in all 142 / 129, 96 scenes of 5.8M
 // 329 / 298. The other walks gain nothing from it (delta of one scene 182 / 182, batched
 // lambda 493 / 502, xsph+normals 323 / 338).
 inline bool far_lists(int64_t n) { return n >= 600000; }
