@@ -213,7 +213,7 @@ __global__ void k_ssfr_bounds(const __grid_constant__ SsfrSplat S, const __grid_
   if (splat_quad(S, smoothPos, g, phase, ii, q)) {
     rect = make_uint2((uint32_t)q.x0 | ((uint32_t)q.x1 << 16), (uint32_t)q.y0 | ((uint32_t)q.y1 << 16));
     const float det = __ldg(&g[ii * 2u + 1u]).z;
-    if (C.on != 0u && fabsf(det) > 1.0e-19f) {
+    if (fabsf(det) > 1.0e-19f) {
       const Ellipsoid E = ellipsoid_of(S, smoothPos, g, ii);
       // the largest singular value of the symmetric G, from above
       float frob = 0.0f, rows = 0.0f;
@@ -300,6 +300,25 @@ __global__ void k_ssfr_depth(const __grid_constant__ SsfrSplat S, const __grid_c
         atomicMin(&key[(size_t)py * width + px], d);
       }
   }
+}
+
+// The depth pass without culling (see ssfr_cull_setup): every splat, one thread each.
+__global__ void k_ssfr_depth_all(const __grid_constant__ SsfrSplat S, const float4* __restrict__ smoothPos,
+                                 const float4* __restrict__ g, const uint4* __restrict__ phase,
+                                 unsigned long long* __restrict__ key, int width) {
+  const uint32_t ii = blockIdx.x * blockDim.x + threadIdx.x;
+  if (ii >= S.count) return;
+  Quad q;
+  if (!splat_quad(S, smoothPos, g, phase, ii, q)) return;
+  const Ellipsoid E = ellipsoid_of(S, smoothPos, g, ii);
+  for (int py = q.y0; py < q.y1; py++)
+    for (int px = q.x0; px < q.x1; px++) {
+      float depth, ez;
+      if (!depth_fragment(S, E, px, py, depth, ez)) continue;
+      if (!(depth < 1.0f)) continue;  // 'less' against the cleared 1.0
+      const unsigned long long k = ((unsigned long long)__float_as_uint(depth) << 32) | ii;
+      atomicMin(&key[(size_t)py * width + px], k);
+    }
 }
 
 __global__ void k_ssfr_depth_resolve(const __grid_constant__ SsfrSplat S, const float4* __restrict__ smoothPos,
@@ -613,7 +632,14 @@ void ssfr_cull_setup(SsfrCull& C, const float* view, const float* proj, const fl
     for (int r = 0; r < 4; r++) b[r] = pv[r] * w[0] + pv[4 + r] * w[1] + pv[8 + r] * w[2] + pv[12 + r] * w[3];
     for (int r = 0; r < 3; r++) ok = ok && near(b[r] / b[3], v[r], r == 2 ? 2e-2 : 1e-3);
   }
-  C.on = ok ? 1u : 0u;
+  // Seen from farther than 270 radii the error bounds leave few splats that surely cover a
+  // pixel (unitErr in k_ssfr_bounds), and the passes before the drawing cost more than they
+  // cull. us a frame at 640 x 480 / 1080p, without and with culling: presets of 30,000 (107
+  // radii away) 246 / 1,045 and 162 / 531, 250,000 (217) 218 / 825 and 154 / 435, 420,000
+  // (258) 230 / 841 and 208 / 640, 500,000 (274) 234 / 861 and 249 / 838, the scene of 264k
+  // with cubes (288) 98 / 188 and 112 / 201.
+  const double radii = distance / std::max(radius, 1e-30);
+  C.on = ok && radii <= 270.0 ? 1u : 0u;
   C.p10 = proj[10];
   C.p14 = proj[14];
   C.transAbs = std::fabs(view[12]) + std::fabs(view[13]) + std::fabs(view[14]);
@@ -637,12 +663,17 @@ void launch_ssfr(const SsfrFrame& f, cudaStream_t st) {
   k_ssfr_body_t<<<mapGrid, tpb, 0, st>>>(f.comp, f.bodies, f.bodyT, f.mapW, f.mapH);
   if (f.depth.count > 0) {
     const int splats = (int)((f.depth.count + tpb - 1) / tpb);
-    cudaMemsetAsync(f.cull.tiles, 0xff, (size_t)f.cull.tilesX * f.cull.tilesY * 4, st);
-    cudaMemsetAsync(f.cull.listed, 0, 4, st);
-    count_launches(3);
-    k_ssfr_bounds<<<splats, tpb, 0, st>>>(f.depth, f.cull, f.smoothPos, f.g, f.phase);
-    k_ssfr_cull<<<splats, tpb, 0, st>>>(f.cull, f.depth.count);
-    k_ssfr_depth<<<148 * 16, tpb, 0, st>>>(f.depth, f.cull, f.smoothPos, f.g, f.depthKey, f.mapW);
+    if (f.cull.on != 0u) {
+      cudaMemsetAsync(f.cull.tiles, 0xff, (size_t)f.cull.tilesX * f.cull.tilesY * 4, st);
+      cudaMemsetAsync(f.cull.listed, 0, 4, st);
+      count_launches(3);
+      k_ssfr_bounds<<<splats, tpb, 0, st>>>(f.depth, f.cull, f.smoothPos, f.g, f.phase);
+      k_ssfr_cull<<<splats, tpb, 0, st>>>(f.cull, f.depth.count);
+      k_ssfr_depth<<<148 * 16, tpb, 0, st>>>(f.depth, f.cull, f.smoothPos, f.g, f.depthKey, f.mapW);
+    } else {
+      count_launches(1);
+      k_ssfr_depth_all<<<splats, tpb, 0, st>>>(f.depth, f.smoothPos, f.g, f.phase, f.depthKey, f.mapW);
+    }
     count_launches(1);
     k_ssfr_thick<<<(f.thick.count + tpb - 1) / tpb, tpb, 0, st>>>(f.thick, f.smoothPos, f.g, f.phase, f.thickAcc,
                                                                   f.thickW);

@@ -159,7 +159,7 @@ struct SsfrComp {  // src/ssfr_composite_wgsl.js:2-26
 // Occlusion culling of the depth splats (kernels_ssfr.cu): tiles of 2^shift pixels that
 // hold the farthest depth a splat is sure to have drawn over the whole tile.
 struct SsfrCull {
-  uint32_t on;              // the matrices are a rigid view and a perspective (ssfr_cull_setup)
+  uint32_t on;              // the splats are culled before they are drawn (ssfr_cull_setup)
   int32_t shift, tilesX, tilesY;
   float p10, p14;           // depth = p14 / distance - p10
   float transAbs, pvAbs;    // sizes of the view's translation and of proj * view, for the error bounds
