@@ -176,8 +176,11 @@ __device__ __forceinline__ float signf(float x) { return x > 0.0f ? 1.0f : (x < 
 // The field's range over blocks of kRangeCells^3 cells, each grown by one cell on every
 // side (minimum, maximum; the whole line when a value is NaN): where a block is all air
 // or all fluid, the march has no crossing to look for and the optical depth no field to
-// interpolate. At 1080p on the 250,000-particle scene marching the field took 1,106 us
-// without them and 573 us with them (the quotients of optical_depth included).
+// interpolate. A positive minimum is lowered by what interpolating the block can round
+// (the march's cubic: 1.2e-4 of the maximum, if every rounding adds up), to 0 where an
+// infinite or overflowing value can turn the result into anything. At 1080p on the
+// 250,000-particle scene marching the field took 1,106 us without them and 573 us with
+// them (the quotients of optical_depth included).
 constexpr int kRangeShift = 2, kRangeCells = 1 << kRangeShift;
 __device__ __forceinline__ float2 range_at(const RayParams& R, const float2* __restrict__ ranges, int cx, int cy,
                                            int cz) {
@@ -209,6 +212,7 @@ __global__ void __launch_bounds__(128) k_ray_ranges(const __grid_constant__ RayP
     lo = fminf(lo, __shfl_xor_sync(0xffffffffu, lo, o));
     hi = fmaxf(hi, __shfl_xor_sync(0xffffffffu, hi, o));
   }
+  if (lo > 0.0f) lo = hi <= 1.0e30f ? fmaxf(lo - 2.0e-4f * hi, 0.0f) : 0.0f;
   if (lane == 0) ranges[b] = make_float2(lo, hi);
 }
 
@@ -301,11 +305,13 @@ __device__ __forceinline__ float optical_depth(const RayParams& R, const float* 
   const float b = fminf(fmaxf(s.t1, 0.0f), tMax);
   if (b <= a) return 0.0f;
   const float dt = (b - a) / (float)R.thickSteps;
-  const float e0 = R.iso * 0.55f, range = R.iso * 1.45f - e0;
+  const float e0 = R.iso * 0.55f, e1 = R.iso * 1.45f, range = e1 - e0;
   // The sample's grid coordinates and its place in the iso band are quotients by the
   // same two numbers in every step: with their reciprocals rounded once (pair_math.cuh),
   // each is the IEEE quotient in three operations instead of ten. Numerators are zero or
-  // far above the underflow limit (differences of values of the scene's size).
+  // far above the underflow limit (differences of values of the scene's size); a field
+  // value above the band counts as its upper end, whose quotient is 1, so that a large or
+  // infinite one does not overflow.
   auto quot = [](float num, float den, float yn) {
     const float qn = num * yn;
     return -fmaf(fmaf(den, qn, num), yn, qn);
@@ -317,7 +323,7 @@ __device__ __forceinline__ float optical_depth(const RayParams& R, const float* 
     // Most samples lie deep in the air or in the fluid: their cell, to within the one
     // cell by which the ranges are grown, is in a block below or above the whole band
     // (by more than three lerps can round), where the smoothstep is exactly 0 or 1.
-    const float air = e0 * 0.9999f, water = R.iso * 1.45f * 1.0001f;
+    const float air = e0 * 0.9999f, water = e1 * 1.0001f;
     const F3 g0 = {-yv * (ro.x - lo.x), -yv * (ro.y - lo.y), -yv * (ro.z - lo.z)};
     const F3 gd = {-yv * rd.x, -yv * rd.y, -yv * rd.z};
     for (int i = 0; i < R.thickSteps; i++) {
@@ -333,7 +339,8 @@ __device__ __forceinline__ float optical_depth(const RayParams& R, const float* 
       }
       const F3 q = {quot(ro.x + rd.x * t - lo.x, R.voxel, yv), quot(ro.y + rd.y * t - lo.y, R.voxel, yv),
                     quot(ro.z + rd.z * t - lo.z, R.voxel, yv)};
-      const float s = clampf(quot(tri_at(R, field, q) - e0, range, yr), 0.0f, 1.0f);
+      const float f = tri_at(R, field, q);
+      const float s = clampf(quot((f > e1 ? e1 : f) - e0, range, yr), 0.0f, 1.0f);
       acc += s * s * (3.0f - 2.0f * s);
     }
   } else {
@@ -341,7 +348,7 @@ __device__ __forceinline__ float optical_depth(const RayParams& R, const float* 
       const float t = a + ((float)i + 0.5f) * dt;
       const F3 q = {(ro.x + rd.x * t - lo.x) / R.voxel, (ro.y + rd.y * t - lo.y) / R.voxel,
                     (ro.z + rd.z * t - lo.z) / R.voxel};
-      acc += smooth(e0, R.iso * 1.45f, tri_at(R, field, q));
+      acc += smooth(e0, e1, tri_at(R, field, q));
     }
   }
   return acc * dt;
