@@ -26,10 +26,11 @@ __device__ __forceinline__ I3 grid_vertex(const MeshParams& M, uint32_t idx, con
 }
 
 // What meshDensity reads of particle j for every vertex around it: its position and
-// (mass / max(rho, rho0 / 2)) * poly6, 0 for a body particle that is skipped (its terms
-// then add +0). Formed once per particle: in the gather below each was recomputed, with
-// its division, for some 500 candidate tests per particle (221 us per field of the
-// 250,000-particle scene on 131 x 131 x 89 vertices).
+// (mass / max(rho, rho0 / 2)) * poly6. A body particle that is skipped counts as infinitely
+// far away, so that it adds nothing whatever its position (NaN among them). Formed once
+// per particle: in the gather below each was recomputed, with its division, for some 500
+// candidate tests per particle (221 us per field of the 250,000-particle scene on
+// 131 x 131 x 89 vertices).
 __global__ void __launch_bounds__(kBlock) k_mesh_weights(const __grid_constant__ MeshParams M,
                                                          const float4* __restrict__ pos,
                                                          const float* __restrict__ rho,
@@ -40,7 +41,7 @@ __global__ void __launch_bounds__(kBlock) k_mesh_weights(const __grid_constant__
   const float4 p = __ldg(&pos[j]);
   const bool skip = M.skipBodies != 0u && __ldg(&body[j]).x != 0u;
   const float vol = M.mass / fmaxf(__ldg(&rho[j]), 0.5f * M.rho0);
-  out[j] = make_float4(p.x, p.y, p.z, skip ? 0.0f : vol * M.poly6);
+  out[j] = skip ? make_float4(INFINITY, INFINITY, INFINITY, 0.0f) : make_float4(p.x, p.y, p.z, vol * M.poly6);
 }
 
 // meshDensity (src/mesh_wgsl.js:23-69). A block takes 8 x 8 x 4 vertices and a warp
