@@ -703,6 +703,9 @@ int p4a_grid_sort(const p4a_grid* grid, int32_t n, float dt, float gravity,
  * tickets start at 1, so tile 0 is never scanned and tile 1 waits on a flag that
  * nothing sets until its limit runs out. Process-wide; restore with (0, 0). */
 int p4a_test_scan_wait(uint32_t spin_limit, int32_t skip_first_tile);
+/* Test hook: the epoch (at most 2^30 - 1) that the handle's last p4a_mesh scanned
+ * with, which the next call counts on from. */
+int p4a_test_mesh_epoch(p4a_sim* sim, uint32_t epoch);
 
 /* ---- operator entry without allocation ---------------------------------- */
 /*

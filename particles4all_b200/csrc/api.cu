@@ -120,7 +120,7 @@ struct p4a_sim {
   uint32_t* meshOffsets = nullptr;                    // [blocks + 1]
   uint2* meshActive = nullptr;                        // [nvox] voxels with triangles (k_mesh_count)
   unsigned long long* meshScan = nullptr;
-  uint32_t* meshTicket = nullptr;
+  uint32_t* meshTicket = nullptr;  // [4]: the scan's ticket and epoch (launch_scan, epoch 0), listed voxels
   uint2* meshVerts = nullptr;
   size_t meshVertCap = 0, meshVoxCap = 0, meshTriCap = 0;
   int fieldSlot = 0, nfieldSlot = 1;  // which of meshField[] hold the fields
@@ -129,7 +129,6 @@ struct p4a_sim {
   double meshOrigin = 0, meshVoxel = 0;
   int64_t meshTris = 0;
   size_t meshBlocks = 0;  // voxel blocks of the last p4a_mesh: meshOffsets[meshBlocks] is its triangle count
-  uint32_t meshEpoch = 0;
   // screen-space fluid rendering (p4a_ssfr)
   std::vector<void*> ssfrAllocs;
   std::vector<void*> ssfrSplats;  // per-splat scratch of the occlusion culling
@@ -1467,10 +1466,9 @@ int p4a_mesh(p4a_sim* s, const p4a_mesh_params* mp, int64_t* triangles) {
     s->nfieldSlot = 0;
   }
   mark(s, PH_MESH_MARCH);
-  uint32_t* activeCount = s->meshTicket + 1;
+  uint32_t* activeCount = s->meshTicket + 2;
   launch_mesh_count(M, buf[0], s->meshCounts, s->meshActive, activeCount, (uint32_t)nvox, st);
-  launch_scan(s->meshCounts, s->meshOffsets, (int)nBlocks, s->meshScan, s->meshTicket, ++s->meshEpoch & 0x3fffffffu,
-              s->d.errorWord, st);
+  launch_scan(s->meshCounts, s->meshOffsets, (int)nBlocks, s->meshScan, s->meshTicket, 0u, s->d.errorWord, st);
   launch_mesh_emit(M, buf[0], buf[s->nfieldSlot], s->meshOffsets, s->meshActive, activeCount, s->meshVerts, st);
   mark(s, PH_END);
   CUDA_TRY(s, cudaGetLastError());
@@ -2104,6 +2102,16 @@ int p4a_test_scan_wait(uint32_t spin_limit, int32_t skip_first_tile) {
   if (skip_first_tile != 0 && skip_first_tile != 1) return P4A_ERR_ARG;
   p4a::g_op_spin_limit.store(spin_limit ? spin_limit : p4a::kScanSpinLimit, std::memory_order_relaxed);
   p4a::g_op_skip_first_tile.store(skip_first_tile, std::memory_order_relaxed);
+  return P4A_OK;
+}
+
+int p4a_test_mesh_epoch(p4a_sim* s, uint32_t epoch) {
+  if (!s || epoch > 0x3fffffffu) return P4A_ERR_ARG;
+  if (!s->meshTicket) return P4A_ERR_STATE;
+  cudaSetDevice(s->device);
+  if (cudaMemcpyAsync(s->meshTicket + 1, &epoch, 4, cudaMemcpyHostToDevice, s->stream) != cudaSuccess ||
+      cudaStreamSynchronize(s->stream) != cudaSuccess)
+    return P4A_ERR_CUDA;
   return P4A_OK;
 }
 
