@@ -1395,14 +1395,14 @@ int p4a_mesh(p4a_sim* s, const p4a_mesh_params* mp, int64_t* triangles) {
       s->meshScan = nullptr;
       s->meshVoxCap = 0;
       CUDA_TRY(s, cudaMalloc((void**)&s->meshCounts, nBlocks * 4));
-      CUDA_TRY(s, cudaMemset(s->meshCounts, 0, nBlocks * 4));
+      CUDA_TRY(s, cudaMemsetAsync(s->meshCounts, 0, nBlocks * 4, s->stream));
       CUDA_TRY(s, cudaMalloc((void**)&s->meshOffsets, (nBlocks + 1) * 4));
       CUDA_TRY(s, cudaMalloc((void**)&s->meshActive, nvox * sizeof(uint2)));
       CUDA_TRY(s, cudaMalloc((void**)&s->meshScan, (size_t)scan_tiles((int)nBlocks) * 8));
-      CUDA_TRY(s, cudaMemset(s->meshScan, 0, (size_t)scan_tiles((int)nBlocks) * 8));
+      CUDA_TRY(s, cudaMemsetAsync(s->meshScan, 0, (size_t)scan_tiles((int)nBlocks) * 8, s->stream));
       if (!s->meshTicket) {
         CUDA_TRY(s, cudaMalloc((void**)&s->meshTicket, 16));
-        CUDA_TRY(s, cudaMemset(s->meshTicket, 0, 16));
+        CUDA_TRY(s, cudaMemsetAsync(s->meshTicket, 0, 16, s->stream));
       }
       s->meshVoxCap = nvox;
     }
@@ -1560,7 +1560,8 @@ int p4a_set_environment(p4a_sim* s, const float* rgb, int32_t width, int32_t hei
   std::vector<uint16_t> host((size_t)6 * size * size * 4);
   build_env_cube(rgb, width, height, size, host.data());
   CUDA_TRY(s, cudaMalloc((void**)&s->envCube, host.size() * 2));
-  CUDA_TRY(s, cudaMemcpy(s->envCube, host.data(), host.size() * 2, cudaMemcpyHostToDevice));
+  CUDA_TRY(s, cudaMemcpyAsync(s->envCube, host.data(), host.size() * 2, cudaMemcpyHostToDevice, s->stream));
+  CUDA_TRY(s, cudaStreamSynchronize(s->stream));  // the host copy goes out of scope
   s->envSize = size;
   return P4A_OK;
 }

@@ -59,9 +59,9 @@ int balloc(p4a_batch* b, T** out, int64_t count) {
   }
   cudaError_t e = cudaMalloc(&p, bytes);
   if (e != cudaSuccess) return bfail(b, P4A_ERR_OOM, "cudaMalloc(%zu): %s", bytes, cudaGetErrorString(e));
-  if ((e = cudaMemset(p, 0, bytes)) != cudaSuccess) {
+  if ((e = cudaMemsetAsync(p, 0, bytes, b->stream)) != cudaSuccess) {
     cudaFree(p);
-    return bfail(b, P4A_ERR_CUDA, "cudaMemset: %s", cudaGetErrorString(e));
+    return bfail(b, P4A_ERR_CUDA, "cudaMemsetAsync: %s", cudaGetErrorString(e));
   }
   b->allocs.push_back(p);
   b->deviceBytes += bytes;
@@ -917,6 +917,8 @@ int p4a_batch_create(int device, const p4a_batch_config* cfg, p4a_batch** out) {
   for (auto& e : b->laneJoin) cudaEventCreateWithFlags(&e, cudaEventDisableTiming);
   const int64_t P = cfg->max_particles, Cc = cfg->max_cells + (int64_t)cfg->max_scenes * (kScanTile + 2);
   int rc = alloc_arenas(b);
+  // the arenas are clear before any other stream (a lane's, a caller's) writes to them
+  if (!rc && cudaStreamSynchronize(b->stream) != cudaSuccess) rc = P4A_ERR_CUDA;
   if (rc) {
     p4a_batch_destroy(b);
     return rc;
