@@ -14,7 +14,7 @@
 // read the other one. Each pass walks lambda's last list, or one it builds with radius
 // h (neighbours.cuh); xsph+normals leaves the list for the tension pass, which walks
 // the same positions. The pair terms run two at a time (pair_math.cuh); parameters
-// outside its ranges take the IEEE operations one entry at a time.
+// outside its ranges take the IEEE operations on the same walk.
 #include <cuda_runtime.h>
 
 #include "neighbours.cuh"

@@ -143,9 +143,11 @@ __device__ __forceinline__ void lambda_body(const SimParams& P, const DevScene& 
       gradSum = fma3(s, rij, gradSum);
     };
     if (count != kListOverflow) {
-      walk1(d.nbList, cap, i, count, [&](uint32_t e) {
-        if ((e & kBoundTag) != 0u) bound(e, __ldg(&d.bsample[e & ~kBoundTag]));
-        else fluid(e, __ldg(&pred[e]));
+      walk2<true, false>(d.nbList, cap, i, count, pred, d.bsample, [&](uint2 e, float4 q0, float4 q1) {
+        if ((e.x & kBoundTag) != 0u) bound(e.x, q0);
+        else fluid(e.x, q0);
+        if ((e.y & kBoundTag) != 0u) bound(e.y, q1);
+        else if (e.y != i) fluid(e.y, q1);
       });
     } else {
       walk_direct<true>(P, w, pi, i, pred, cs, bcs, d.bsample, fluid, bound);
@@ -259,9 +261,11 @@ __device__ __forceinline__ void delta_body(const SimParams& P, const DevScene& d
       dB = fma3(coef, rij, dB);
     };
     if (count != kListOverflow) {
-      walk1(d.nbList, d.cap, i, count, [&](uint32_t e) {
-        if ((e & kBoundTag) != 0u) bound(e, __ldg(&d.bsample[e & ~kBoundTag]));
-        else fluid(e, __ldg(&pl[e]));
+      walk2<true, false>(d.nbList, d.cap, i, count, pl, d.bsample, [&](uint2 e, float4 q0, float4 q1) {
+        if ((e.x & kBoundTag) != 0u) bound(e.x, q0);
+        else fluid(e.x, q0);
+        if ((e.y & kBoundTag) != 0u) bound(e.y, q1);
+        else if (e.y != i) fluid(e.y, q1);
       });
     } else {
       const RowWalk w(P, pi);

@@ -323,16 +323,6 @@ __device__ __forceinline__ void walk2(const uint32_t* list, uint32_t cap, uint32
   }
 }
 
-// The entries of a list one at a time: visit(entry). For parameters outside the ranges
-// of the pair arithmetic (pair_math_ranges).
-template <class F>
-__device__ __forceinline__ void walk1(const uint32_t* list, uint32_t cap, uint32_t i, uint32_t count,
-                                      F&& visit) {
-  count &= kCountMask;
-#pragma unroll 1
-  for (uint32_t k = 0; k < count; k++) visit(list[list_at(k, cap, i)]);
-}
-
 // The reference's direct loop (particles whose list overflowed): every candidate
 // j != self of the nine rows with r^2 < h^2 (the particle itself contributes to
 // no pass), then, when B, the row's boundary samples with 1e-12 <= r^2 < h^2. fsrc
@@ -406,7 +396,7 @@ __device__ __forceinline__ void walk2g(const uint32_t* list, uint32_t cap, uint3
   }
 }
 
-// The fluid-only passes one entry at a time: visit(pred[j], gsrc[j]) of every listed
+// The fluid-only passes with the IEEE operations: visit(pred[j], gsrc[j]) of every listed
 // fluid entry, or of the reference's direct loop for an overflowed list.
 template <class F>
 __device__ __forceinline__ void walk_fluid(const SimParams& P, const RowWalk& w, uint32_t i, F3 pi,
@@ -418,8 +408,9 @@ __device__ __forceinline__ void walk_fluid(const SimParams& P, const RowWalk& w,
                        [&](uint32_t j, float4 q) { visit(q, __ldg(&gsrc[j])); }, [](uint32_t, float4) {});
     return;
   }
-  walk1(list, cap, i, count, [&](uint32_t e) {
-    if ((e & kBoundTag) == 0u) visit(__ldg(&pred[e]), __ldg(&gsrc[e]));
+  walk2g(list, cap, i, count, pred, gsrc, [&](uint32_t j0, uint32_t j1, float4 q0, float4 q1, float4 g0, float4 g1) {
+    if (j0 != i) visit(q0, g0);
+    if (j1 != i) visit(q1, g1);
   });
 }
 
