@@ -1606,13 +1606,15 @@ int p4a_ssfr(p4a_sim* s, const p4a_ssfr_params* sp, const float* bodies, int32_t
     s->ssfrMapW = s->ssfrMapH = s->ssfrThW = s->ssfrThH = s->ssfrW = s->ssfrH = 0;
     const size_t mapN = (size_t)mapW * mapH, thN = (size_t)tw * th;
     int rc;
-    if ((rc = dalloc(s, s->ssfrAllocs, &F.depthKey, mapN)) || (rc = dalloc(s, s->ssfrAllocs, &F.thickAcc, thN)) ||
+    // the keys, and behind them the culling's tiles: both start as all ones
+    if ((rc = dalloc(s, s->ssfrAllocs, &F.depthKey, mapN + (mapN + 1) / 2)) || (rc = dalloc(s, s->ssfrAllocs, &F.thickAcc, thN)) ||
         (rc = dalloc(s, s->ssfrAllocs, &F.eyeZ[0], mapN)) || (rc = dalloc(s, s->ssfrAllocs, &F.eyeZ[1], mapN)) ||
         (rc = dalloc(s, s->ssfrAllocs, &F.raw, mapN)) || (rc = dalloc(s, s->ssfrAllocs, &F.thickMap, thN)) ||
         (rc = dalloc(s, s->ssfrAllocs, &F.thickTmp, thN)) || (rc = dalloc(s, s->ssfrAllocs, &F.bodyT, mapN)) ||
         (rc = dalloc(s, s->ssfrAllocs, &F.image, (size_t)q.width * q.height)) ||
-        (rc = dalloc(s, s->ssfrAllocs, &F.cull.tiles, mapN)) || (rc = dalloc(s, s->ssfrAllocs, &F.cull.listed, 4)))
+        (rc = dalloc(s, s->ssfrAllocs, &F.cull.listed, 4)))
       return rc;
+    F.cull.tiles = reinterpret_cast<uint32_t*>(F.depthKey + mapN);
     s->ssfrMapW = mapW;
     s->ssfrMapH = mapH;
     s->ssfrThW = tw;
@@ -1680,7 +1682,7 @@ int p4a_ssfr(p4a_sim* s, const p4a_ssfr_params* sp, const float* bodies, int32_t
   splat(F.thick, tw, th, thickRadius, 0.0);
   double toScene = 0.0;  // from the eye to the middle of the box
   for (int k = 0; k < 3; k++) toScene = std::hypot(toScene, q.eye[k] - 0.5 * s->params.box[k]);
-  ssfr_cull_setup(F.cull, q.view, q.proj, q.inv_view_proj, mapW, mapH, q.splat_radius * spacing, toScene);
+  ssfr_cull_setup(F.cull, q.view, q.proj, q.inv_view_proj, mapW, mapH, s->n, q.splat_radius * spacing, toScene);
   // thickness blur (src/ssfr.js:227-233)
   const int blurSize = q.thickness_filter_size == 0 ? 0
                        : (tw < mapW ? std::max(1, q.thickness_filter_size >> 1) : q.thickness_filter_size);

@@ -206,6 +206,7 @@ __global__ void k_ssfr_bounds(const __grid_constant__ SsfrSplat S, const __grid_
                               const float4* __restrict__ smoothPos, const float4* __restrict__ g,
                               const uint4* __restrict__ phase) {
   const uint32_t ii = blockIdx.x * blockDim.x + threadIdx.x;
+  if (ii == 0u) *C.listed = 0u;  // for the cull pass
   if (ii >= S.count) return;
   Quad q;
   uint2 rect = make_uint2(0u, 0u);
@@ -605,7 +606,7 @@ __global__ void k_ssfr_composite(const __grid_constant__ SsfrComp C, const float
 }  // namespace
 
 void ssfr_cull_setup(SsfrCull& C, const float* view, const float* proj, const float* ivp, int mapW, int mapH,
-                     double radius, double distance) {
+                     int64_t splats, double radius, double distance) {
   auto near = [](double a, double b, double tol) { return std::fabs(a - b) <= tol; };
   bool ok = proj[0] > 0.0f && proj[5] > 0.0f && proj[11] == -1.0f && proj[14] < 0.0f;
   for (int k : {1, 2, 3, 4, 6, 7, 8, 9, 12, 13, 15}) ok = ok && proj[k] == 0.0f;
@@ -638,15 +639,20 @@ void ssfr_cull_setup(SsfrCull& C, const float* view, const float* proj, const fl
   // radii away) 246 / 1,045 and 162 / 531, 250,000 (217) 218 / 825 and 154 / 435, 420,000
   // (258) 230 / 841 and 208 / 640, 500,000 (274) 234 / 861 and 249 / 838, the scene of 264k
   // with cubes (288) 98 / 188 and 112 / 201.
-  const double radii = distance / std::max(radius, 1e-30);
-  C.on = ok && radii <= 270.0 ? 1u : 0u;
+  // Splats of a few pixels are drawn by one thread each before the two passes have run, unless
+  // there are very many: blocks of 4,096 / 32,768, 144 radii away, at 320 x 240 (radius 2.0
+  // pixels) 127 / 128 us a frame without and 131 / 133 with culling, three streams side by
+  // side 57 / 57 and 63 / 62; at 640 x 480 (4.0 pixels) 175 / 201 and 153 / 175, side by side
+  // 57 / 77 and 62 / 67; 110,592 of 2.7 pixels 163 and 154, 63 and 64; the 420,000 above have
+  // 2.2 pixels at 640 x 480.
+  const double radii = distance / std::max(radius, 1e-30), px = radius * proj[5] * 0.5 * mapH / std::max(distance, 1e-6);
+  C.on = ok && radii <= 270.0 && (px >= 2.5 || (double)splats * px * px >= 1.0e6) ? 1u : 0u;
   C.p10 = proj[10];
   C.p14 = proj[14];
   C.transAbs = std::fabs(view[12]) + std::fabs(view[13]) + std::fabs(view[14]);
   C.pvAbs = (float)pvAbs;
   // tiles of about 0.7 of the splats' radius: a splat then surely covers one or two, and
   // few tiles are read per splat (any size gives the same image)
-  const double px = radius * proj[5] * 0.5 * mapH / std::max(distance, 1e-6);
   C.shift = 0;
   while (C.shift < 5 && (double)(2 << C.shift) <= 0.75 * px) C.shift++;
   C.tilesX = ((mapW - 1) >> C.shift) + 1;
@@ -656,7 +662,8 @@ void ssfr_cull_setup(SsfrCull& C, const float* view, const float* proj, const fl
 void launch_ssfr(const SsfrFrame& f, cudaStream_t st) {
   const int tpb = 128;
   const int64_t mapN = (int64_t)f.mapW * f.mapH, thN = (int64_t)f.thickW * f.thickH;
-  cudaMemsetAsync(f.depthKey, 0xff, (size_t)mapN * 8, st);
+  const size_t tiles = f.cull.on != 0u ? (size_t)f.cull.tilesX * f.cull.tilesY : 0;
+  cudaMemsetAsync(f.depthKey, 0xff, (size_t)mapN * 8 + tiles * 4, st);  // keys and, behind them, tiles
   cudaMemsetAsync(f.thickAcc, 0, (size_t)thN * 8, st);
   const dim3 mapGrid((f.mapW + tpb - 1) / tpb, f.mapH), thGrid((f.thickW + tpb - 1) / tpb, f.thickH);
   count_launches(1);
@@ -664,8 +671,6 @@ void launch_ssfr(const SsfrFrame& f, cudaStream_t st) {
   if (f.depth.count > 0) {
     const int splats = (int)((f.depth.count + tpb - 1) / tpb);
     if (f.cull.on != 0u) {
-      cudaMemsetAsync(f.cull.tiles, 0xff, (size_t)f.cull.tilesX * f.cull.tilesY * 4, st);
-      cudaMemsetAsync(f.cull.listed, 0, 4, st);
       count_launches(3);
       k_ssfr_bounds<<<splats, tpb, 0, st>>>(f.depth, f.cull, f.smoothPos, f.g, f.phase);
       k_ssfr_cull<<<splats, tpb, 0, st>>>(f.cull, f.depth.count);

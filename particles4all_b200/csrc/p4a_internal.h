@@ -174,9 +174,10 @@ struct SsfrCull {
   uint32_t* tiles;          // [tilesX * tilesY] float bits
 };
 // Sets on, shift, the tile counts and the constants from the camera (double math);
-// `radius` is the splats' radius and `distance` the scene's distance, which set the tile size.
+// `radius` is the splats' radius and `distance` the scene's distance, which set the tile size;
+// they and the count of splats decide whether culling pays.
 void ssfr_cull_setup(SsfrCull& C, const float* view, const float* proj, const float* ivp, int mapW, int mapH,
-                     double radius, double distance);
+                     int64_t splats, double radius, double distance);
 
 struct SsfrFrame {
   SsfrSplat depth, thick;
@@ -191,7 +192,7 @@ struct SsfrFrame {
   const float4* g;
   const uint4* phase;
   const float4* bodies;
-  unsigned long long* depthKey;  // [mapW * mapH]
+  unsigned long long* depthKey;  // [mapW * mapH], with cull.tiles behind it
   unsigned long long* thickAcc;  // [thickW * thickH]
   float* eyeZ[2];                // [mapW * mapH] ping-pong
   float* raw;                    // [mapW * mapH] unfiltered eye-space z
