@@ -706,6 +706,12 @@ int p4a_test_scan_wait(uint32_t spin_limit, int32_t skip_first_tile);
 /* Test hook: the epoch (at most 2^30 - 1) that the handle's last p4a_mesh scanned
  * with, which the next call counts on from. */
 int p4a_test_mesh_epoch(p4a_sim* sim, uint32_t epoch);
+/* Test hook: checks the neighbour passes' square roots, reciprocals and quotients
+ * against the IEEE operations on the current device, for every float in [lo, hi)
+ * (within [2^-100, 2^100]). counts: arguments whose root differs, whose reciprocal
+ * differs, whose root's reciprocal is not the rounded one, and, for those, the
+ * quotients by the root that differ, over the 2^23 numerators from `numerator` on. */
+int p4a_test_pair_math(float lo, float hi, float numerator, uint64_t counts[4]);
 
 /* ---- operator entry without allocation ---------------------------------- */
 /*

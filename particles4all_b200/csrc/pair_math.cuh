@@ -8,11 +8,12 @@
 // s = g + h (x - g g) is the rounded root; a Newton step turns y into the reciprocal
 // of s; and a quotient a / s is q = a y corrected once by the exact remainder,
 // q + y (a - s q), which is the rounded quotient whenever y is the rounded reciprocal.
-// Checked on the device over every float in [2^-60, 2^60]: every root is sqrtf's and
-// every recip() is the rounded reciprocal; the reciprocal of a root is the rounded one
-// but for a few dozen roots per binade, and for each of those the quotients of all
-// 2^23 numerators equal the IEEE division's (the approximation is taken one ulp up
-// because the all-ones root fails that check without it).
+// Checked on the device (p4a_test_pair_math) over every float: in [2^-96, 2^100] every
+// root is sqrtf's, in [2^-60, 2^60] every recip() is the rounded reciprocal; the
+// reciprocal of a root is the rounded one but for 10 or 24 roots per binade, and for each
+// of those the quotients of all 2^23 numerators equal the IEEE division's (the
+// approximation is taken one ulp up because the all-ones root fails that check without
+// it).
 //
 // Blackwell's packed f32x2 instructions do two independent binary32 operations in one
 // issue slot, each rounded as the scalar instruction rounds it (the FMA pipe is as
