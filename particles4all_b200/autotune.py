@@ -3,8 +3,9 @@
 The library compiles lambda, delta, xsph+normals and the anisotropic pass in
 several launch shapes (threads per block x minimum resident blocks per SM, i.e.
 particles per block and the register budget); all shapes compute the same bits.
-For every size bucket this steps a seeded dam-break scene of that size (the
-served workload's scenes, with surface tension on so the normals pass runs),
+For every size bucket whose scenes launch them this steps a seeded dam-break scene of
+that size (the served workload's scenes, with surface tension on so the normals pass
+runs),
 frame by frame with the shapes of one kernel taking turns, and reads that
 kernel's device time per launch from the library's per-kernel CUDA events. The
 fastest shape per (kernel, bucket) goes into the library's table (p4a_tune_set)
@@ -33,8 +34,11 @@ DEFAULT_PATH = os.path.join(HERE, "tuning.json")
 KERNELS = {"lambda": 0, "delta": 1, "xsph_normals": 2, "aniso": 3}
 BATCHED = {"lambda_batched": 4, "delta_batched": 5, "xsph_normals_batched": 6}
 PROFILE_NAME = {"lambda_batched": "lambda", "delta_batched": "delta", "xsph_normals_batched": "xsph_normals"}
+# plain scenes of up to this many particles take the passes with a group of lanes per
+# particle (csrc/api.cu group_lanes), which have no launch shapes
+GROUPED = 20_000
 # bucket upper bounds (particles) and the scene size measured for each
-BUCKETS = [(24_000, 12_000), (96_000, 48_000), (384_000, 192_000), (1_536_000, 768_000), (1 << 40, 2_000_000)]
+BUCKETS = [(GROUPED, 12_000), (24_000, 22_000), (96_000, 48_000), (384_000, 192_000), (1_536_000, 768_000), (1 << 40, 2_000_000)]
 # batched buckets: upper bound of a frame's total particles and the scene count of
 # the seeded mix measured for it (96 scenes: about 6.0 M particles)
 BATCH_BUCKETS = [(3_000_000, 24), (1 << 40, 96)]
@@ -161,6 +165,9 @@ def tune_batched(result, L, buckets=BATCH_BUCKETS, frames=4, log=print):
 
 def tune(buckets=BUCKETS, frames=6, path=DEFAULT_PATH, log=print, batch_buckets=BATCH_BUCKETS):
     from ._lib import lib
+    for bound, n in buckets:
+        if (n > GROUPED) != (bound > GROUPED):
+            raise ValueError(f"bucket up to {bound} particles: a scene of {n} takes other passes")
     L = lib()
     L.p4a_tune_clear(-1)
     result = {"kernels": {k: [] for k in KERNELS}, "measured": {}, "shapes": {}}
@@ -175,7 +182,8 @@ def tune(buckets=BUCKETS, frames=6, path=DEFAULT_PATH, log=print, batch_buckets=
             sim.aniso(aniso)
         run, step = _sim_profile(sim, aniso)
         per = {}
-        for name, k in KERNELS.items():
+        tuned = KERNELS if bound > GROUPED else {"aniso": KERNELS["aniso"]}
+        for name, k in tuned.items():
             variants = list(range(len(result["shapes"][name])))
             times = interleaved(step, run, L, k, name, variants, frames)
             best = min(range(len(times)), key=times.__getitem__)
@@ -185,7 +193,7 @@ def tune(buckets=BUCKETS, frames=6, path=DEFAULT_PATH, log=print, batch_buckets=
             log(f"n={real_n:>9} {name:13s} " + " ".join(f"{x * 1e3:7.1f}" for x in times) + f"  -> {best}")
         sim.close()
         result["measured"][str(real_n)] = per
-        for name in KERNELS:
+        for name in tuned:
             result["kernels"][name].append([bound, per[name]["best"]])
     if batch_buckets:
         L.p4a_tune_clear(-1)
