@@ -96,6 +96,8 @@ struct p4a_sim {
   int heldBody = -1;
   double heldTarget[3] = {0, 0, 0}, heldRate = 10, heldLimit = 4;
   SimParams P{};
+  bool boundaryOut = false;  // a caller has the device pointer of bpos or bpsi and may write through it
+  bool psiOut = false;       // a caller has written psi or has its pointer: any values, any range
   FrameGraph frames[kFrameGraphs];  // p4a_step
   uint64_t frameUse = 0;
   cudaStream_t captureStream = nullptr;
@@ -318,7 +320,7 @@ void pack_params(p4a_sim* s, double dt) {
   F.skinH2 = (float)((h + kSkin * h) * (h + kSkin * h));
   F.skinHalf = (float)((kSkin * h - 1e-4 * h) * 0.5);
   F.volSpiky = F.volume * F.spikyGrad;
-  F.pairMath = pair_math_ranges(F);
+  F.pairMath = s->psiOut ? 0u : pair_math_ranges(F);  // whose bounds are the library's own psi
 }
 
 // Lanes per particle of the neighbour passes of a plain scene (0: one thread per
@@ -370,8 +372,18 @@ int upload_boundary(p4a_sim* s) {
                               cudaMemcpyHostToDevice, s->stream));
   CUDA_TRY(s, cudaStreamSynchronize(s->stream));  // host vectors go out of scope
   s->nBoundary = nb;
+  s->boundaryOut = s->psiOut = false;
   return P4A_OK;
 }
+
+// Brings the walks' copy of the boundary samples up to date: after a p4a_write of theirs,
+// and before every frame once p4a_buffer has handed out one of their device pointers.
+void pack_boundary(p4a_sim* s) {
+  if (s->nBoundary < 1) return;
+  count_launches(1);
+  launch_pack_boundary(s->d, (uint32_t)s->nBoundary, s->stream);
+}
+bool is_boundary(int32_t id) { return id == P4A_BUF_BPOS || id == P4A_BUF_BPSI; }
 
 // The grid pass at parity `par` into parity par^1 (src/sim.js:473-492).
 void grid_pass(p4a_sim* s, int par) {
@@ -990,6 +1002,7 @@ int p4a_step(p4a_sim* s, double frameDt, int32_t* substeps_out) {
   SimParams& P = s->P;
   cudaStream_t st = s->stream;
   const bool dragging = s->heldBody >= 1 && s->nBodyParts > 0;
+  if (s->boundaryOut) pack_boundary(s);
   FrameGraph* f = dragging || s->prof ? nullptr : frame_graph(s, sub);
   if (f) {
     CUDA_TRY(s, cudaGraphLaunch(f->exec, st));
@@ -1176,6 +1189,8 @@ int p4a_buffer(p4a_sim* s, int32_t id, int32_t which, void** dptr, size_t* bytes
   size_t b = 0;
   const int rc = buffer_ptr(s, id, which, dptr, &b);
   if (bytes) *bytes = b;
+  if (!rc && is_boundary(id)) s->boundaryOut = true;
+  if (!rc && id == P4A_BUF_BPSI) s->psiOut = true;
   return rc;
 }
 
@@ -1240,6 +1255,8 @@ int p4a_write(p4a_sim* s, int32_t id, int32_t which, const void* host, size_t of
   after_reads(s, buf_bit(id));
   s->sortedMoves = false;
   CUDA_TRY(s, cudaMemcpyAsync((char*)p + offset, host, bytes, cudaMemcpyHostToDevice, s->stream));
+  if (is_boundary(id)) pack_boundary(s);
+  if (id == P4A_BUF_BPSI) s->psiOut = true;
   CUDA_TRY(s, cudaStreamSynchronize(s->stream));
   return P4A_OK;
 }

@@ -235,6 +235,19 @@ void launch_resize(uint32_t n, float4* pos, const float oldSize[3], const float 
                                          F3{clampMax[0], clampMax[1], clampMax[2]});
 }
 
+// The walks' copy of the boundary samples (DevScene::bsample) from the buffers that a
+// caller reads and writes.
+__global__ void __launch_bounds__(kBlock) k_pack_boundary(const float4* __restrict__ pos, const float* __restrict__ psi,
+                                                          uint32_t n, float4* __restrict__ out) {
+  const uint32_t k = blockIdx.x * kBlock + threadIdx.x;
+  if (k >= n) return;
+  const float4 p = __ldg(&pos[k]);
+  out[k] = make_float4(p.x, p.y, p.z, __ldg(&psi[k]));
+}
+void launch_pack_boundary(const DevScene& d, uint32_t n, cudaStream_t st) {
+  k_pack_boundary<<<groups(n), kBlock, 0, st>>>(d.bpos, d.bpsi, n, d.bsample);
+}
+
 template <int TB, int MB, bool FAST>
 __global__ void __launch_bounds__(TB, MB) k_aniso(const __grid_constant__ AnisoParams A,
                                                   const float4* __restrict__ pos,

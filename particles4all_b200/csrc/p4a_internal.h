@@ -255,9 +255,10 @@ struct DevScene {
   uint32_t* unordered;
   unsigned long long* scanState;  // epoch-tagged tile states
   uint32_t* scanTicket;
-  float4* bpos;         // plain scenes only, with bpsi: the buffers p4a_read returns
+  float4* bpos;         // plain scenes only, with bpsi: the buffers that callers read and write
   float* bpsi;
-  float4* bsample;      // (position, psi) of each boundary sample: one gather in the walks
+  float4* bsample;      // (position, psi) of each boundary sample: one gather in the walks;
+                        // in plain scenes a copy of bpos and bpsi (pack_boundary in api.cu)
   uint32_t* bcellStart;
   int32_t* bodyAccum;   // 4 per body
   int32_t* bodyCov;     // 9 per body
@@ -435,6 +436,7 @@ void launch_body_drag(const DevScene& d, float4* vel, const uint4* body, uint32_
 void launch_impulse(uint32_t n, const float4* pos, float4* vel, const float origin[3],
                     const float dir[3], const float impulse[3], float radius, float speedLimit,
                     cudaStream_t st);
+void launch_pack_boundary(const DevScene& d, uint32_t n, cudaStream_t st);
 void launch_resize(uint32_t n, float4* pos, const float oldSize[3], const float newSize[3],
                    const float clampMin[3], const float clampMax[3], cudaStream_t st);
 void launch_aniso(const AnisoParams& A, const float4* pos, const uint32_t* cellStart,
