@@ -305,13 +305,13 @@ __device__ __forceinline__ float optical_depth(const RayParams& R, const float* 
   const float b = fminf(fmaxf(s.t1, 0.0f), tMax);
   if (b <= a) return 0.0f;
   const float dt = (b - a) / (float)R.thickSteps;
-  const float e0 = R.iso * 0.55f, e1 = R.iso * 1.45f, range = e1 - e0;
+  const float e0 = R.iso * 0.55f, range = R.iso * 1.45f - e0;
   // The sample's grid coordinates and its place in the iso band are quotients by the
   // same two numbers in every step: with their reciprocals rounded once (pair_math.cuh),
   // each is the IEEE quotient in three operations instead of ten. Numerators are zero or
   // far above the underflow limit (differences of values of the scene's size); a field
   // value above the band counts as its upper end, whose quotient is 1, so that a large or
-  // infinite one does not overflow.
+  // infinite one does not overflow (and NaN stays NaN, which counts as 0).
   auto quot = [](float num, float den, float yn) {
     const float qn = num * yn;
     return -fmaf(fmaf(den, qn, num), yn, qn);
@@ -323,7 +323,7 @@ __device__ __forceinline__ float optical_depth(const RayParams& R, const float* 
     // Most samples lie deep in the air or in the fluid: their cell, to within the one
     // cell by which the ranges are grown, is in a block below or above the whole band
     // (by more than three lerps can round), where the smoothstep is exactly 0 or 1.
-    const float air = e0 * 0.9999f, water = e1 * 1.0001f;
+    const float air = e0 * 0.9999f, water = R.iso * 1.45f * 1.0001f;
     const F3 g0 = {-yv * (ro.x - lo.x), -yv * (ro.y - lo.y), -yv * (ro.z - lo.z)};
     const F3 gd = {-yv * rd.x, -yv * rd.y, -yv * rd.z};
     for (int i = 0; i < R.thickSteps; i++) {
@@ -339,8 +339,13 @@ __device__ __forceinline__ float optical_depth(const RayParams& R, const float* 
       }
       const F3 q = {quot(ro.x + rd.x * t - lo.x, R.voxel, yv), quot(ro.y + rd.y * t - lo.y, R.voxel, yv),
                     quot(ro.z + rd.z * t - lo.z, R.voxel, yv)};
-      const float f = tri_at(R, field, q);
-      const float s = clampf(quot((f > e1 ? e1 : f) - e0, range, yr), 0.0f, 1.0f);
+      // the quotient as by quot, clamped to [0, 1] (NaN to 0) by its last operation: with
+      // the clamp after it and the select of large values 281.3 us a mesh view of the
+      // 250,000-particle scene, 279.8 like this
+      float num, s;
+      asm("min.NaN.f32 %0, %1, %2;" : "=f"(num) : "f"(tri_at(R, field, q) - e0), "f"(range));
+      const float qn = num * yr;
+      asm("fma.rn.sat.f32 %0, %1, %2, %3;" : "=f"(s) : "f"(fmaf(range, qn, num)), "f"(-yr), "f"(-qn));
       acc += s * s * (3.0f - 2.0f * s);
     }
   } else {
@@ -348,7 +353,7 @@ __device__ __forceinline__ float optical_depth(const RayParams& R, const float* 
       const float t = a + ((float)i + 0.5f) * dt;
       const F3 q = {(ro.x + rd.x * t - lo.x) / R.voxel, (ro.y + rd.y * t - lo.y) / R.voxel,
                     (ro.z + rd.z * t - lo.z) / R.voxel};
-      acc += smooth(e0, e1, tri_at(R, field, q));
+      acc += smooth(e0, R.iso * 1.45f, tri_at(R, field, q));
     }
   }
   return acc * dt;
