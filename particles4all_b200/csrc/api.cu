@@ -326,16 +326,20 @@ void pack_params(p4a_sim* s, double dt) {
 // Lanes per particle of the neighbour passes of a plain scene (0: one thread per
 // particle). A group shortens each particle's chain of dependent loads but issues more
 // instructions, so it gains while the GPU has idle schedulers, also with other scenes on
-// other streams. us per frame, one scene alone / a frame of three scenes on three streams,
-// with one thread, 16 and 8 lanes per particle, dam break (D, 2 substeps of 4 iterations)
-// and the sloshing preset (P, 4 of 4, lists rebuilt in most iterations):
-//   D  2,197: 309/125 187/86  192/89      P  2,500: 1397/558  597/252  638/271
-//   D  4,000: 342/137 201/94  212/93      P  5,000: 1448/592  640/280  673/292
-//   D  8,000: 356/145 225/109 230/105     P  8,000: 1479/603  683/331  716/318
-//   D 16,000: 376/156 293/149 257/133     P 16,000: 1494/629  963/502  822/435
-//   D 24,000: 387/162 356/197 326/172     P 24,000: 1604/673 1162/691 1083/593
-//   D 32,768: 392/169 415/255 362/214     P 40,000: 1713/774 1593/1093 1411/911
-// Past 20,000 particles the lone scene still gains but scenes side by side lose.
+// other streams. us per frame, one scene alone with the host's wait / a frame of three
+// scenes on three streams, with one thread, 16 and 8 lanes per particle, dam break (D, 2
+// substeps of 4 iterations) and the sloshing preset (P, 4 of 4, lists rebuilt in most
+// iterations), frames replayed as graphs:
+//   D  2,197: 262/85  167/49  168/55      P  2,580: 1015/355 520/178  556/193
+//   D  4,096: 264/87  176/58  176/61      P  5,200: 1051/376 557/207  588/214
+//   D  5,832: 291/97  191/66  192/68      P  6,224: 1080/369 561/222  595/226
+//   D  8,000: 304/102 201/77  201/75      P  8,348: 1093/385 608/256  616/249
+//   D 15,625: 326/111 266/120 244/108     P 16,692: 1079/392 856/437  719/366
+//   D 19,683: 325/117 300/142 266/126     P 20,774: 1076/404 939/538  845/444
+//   D 24,389: 331/121 332/170 307/149     P 24,976: 1102/415 1025/630 953/519
+//   D 32,768: 350/124 387/218 337/187     P 33,348: 1126/444 1236/815 1061/667
+// Around 20,000 particles the lone scene gains 18-22 % and three side by side lose 7-10 %;
+// past it the loss soon outweighs the gain.
 constexpr int kGroup16 = 6000, kGroup8 = 20000;
 int group_lanes(int n) { return n <= kGroup16 ? 16 : n <= kGroup8 ? 8 : 0; }
 

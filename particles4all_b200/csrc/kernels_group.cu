@@ -12,8 +12,8 @@
 // addition is fma(1, b, acc); an entry that does not contribute has a zero term, which
 // leaves every sum as it is). Roots and quotients are those of pair_math.cuh (FAST), or
 // the IEEE operations for parameters outside its ranges. Bound by the latency of those
-// chains, whose length falls with G; a frame of 2,197 particles takes 187 us with 16 lanes
-// and 309 us with one thread per particle (group_lanes in api.cu has the other sizes).
+// chains, whose length falls with G; a frame of 2,197 particles takes 167 us with 16 lanes
+// and 262 us with one thread per particle (group_lanes in api.cu has the other sizes).
 // 32 lanes gain 3 % more below 3,000 particles and lose above: not built.
 #include <cuda_runtime.h>
 

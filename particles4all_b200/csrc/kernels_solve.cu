@@ -31,12 +31,14 @@ namespace p4a {
 
 // One list walk of lambda, two entries at a time; B: the list holds boundary samples
 // (a fluid entry then takes the same path with its own coefficients selected, so that a
-// warp at a wall runs every pair once and not once per kind). The walks are bound by
-// issue slots (77 % of them busy, 80 warp-instructions per entry, a quarter of those in
-// the range tests of an IEEE root and division); with the packed pair arithmetic lambda
-// takes 525 us per launch on the 96-scene mix in halves (728 us one entry at a time with
-// the IEEE operations), delta 327 us (426 us); on the large scene 269 us (289 us) and
-// 178 us (232 us).
+// warp at a wall runs every pair once and not once per kind). One entry at a time with the
+// IEEE operations the walks were bound by issue slots (77 % of them busy, 80
+// warp-instructions per entry, a quarter of those in the range tests of a root and a
+// division): lambda took 728 us per launch on the 96-scene mix in halves, delta 426 us, on
+// the large scene 289 and 232 us. With the packed pair arithmetic 525 and 327 us, 284 and
+// 182 us; with the builds of neighbours.cuh and the prefetch of far_lists 492 and 297 us,
+// 260 and 182 us. What bounds them now is the latency of the gathers (62 % of the slots, 49 %
+// of the warps).
 template <bool B, bool FAR>
 __device__ __forceinline__ void lambda_walk(const SimParams& P, const DevScene& d, uint32_t i, uint32_t count, F3 pi,
                                             const float4* __restrict__ pred, float& rho, F3& gradSum,
