@@ -220,6 +220,7 @@ struct March {
   float t;
   F3 pos, nrm;
 };
+template <bool RANGES>
 __device__ __forceinline__ March march(const RayParams& R, const float* __restrict__ field,
                                        const float2* __restrict__ ranges, const float4* __restrict__ bdata, F3 ro,
                                        F3 rd, float tStart, float tEnd) {
@@ -255,7 +256,8 @@ __device__ __forceinline__ March march(const RayParams& R, const float* __restri
   for (int i = 0; i < 4096; i++) {
     const float tNext = fminf(fminf(tMax[0], tMax[1]), tMax[2]);
     const float segEnd = fminf(tNext, tEnd);
-    const float2 range = range_at(R, ranges, c[0], c[1], c[2]);
+    float2 range = make_float2(-1.0f, 0.0f);
+    if constexpr (RANGES) range = range_at(R, ranges, c[0], c[1], c[2]);
     if (segEnd > t && !(R.iso > 0.0f && range.x >= 0.0f && (range.y <= below || range.x >= above))) {
       const Cell k = cell_at(R, field, c[0], c[1], c[2]);
       const F3 u0 = {g0.x + gd.x * t - (float)c[0], g0.y + gd.y * t - (float)c[1], g0.z + gd.z * t - (float)c[2]};
@@ -294,6 +296,7 @@ __device__ __forceinline__ March march(const RayParams& R, const float* __restri
   }
   return out;
 }
+template <bool RANGES>
 __device__ __forceinline__ float optical_depth(const RayParams& R, const float* __restrict__ field,
                                                const float2* __restrict__ ranges, F3 ro, F3 rd, float tMax) {
   const F3 lo = f3(R.gridOrigin);
@@ -328,7 +331,7 @@ __device__ __forceinline__ float optical_depth(const RayParams& R, const float* 
     const F3 gd = {-yv * rd.x, -yv * rd.y, -yv * rd.z};
     for (int i = 0; i < R.thickSteps; i++) {
       const float t = a + ((float)i + 0.5f) * dt;
-      if (ranges != nullptr) {
+      if constexpr (RANGES) {
         const float2 band = range_at(R, ranges, (int)floorf(fmaf(gd.x, t, g0.x)), (int)floorf(fmaf(gd.y, t, g0.y)),
                                      (int)floorf(fmaf(gd.z, t, g0.z)));
         if (band.y <= air) continue;
@@ -530,6 +533,7 @@ __global__ void k_surf_resolve(const __grid_constant__ RayParams R, const __grid
   surfN[o] = nn;
 }
 
+template <bool RANGES>
 __global__ void __launch_bounds__(128, 8) k_ray(const __grid_constant__ RayParams R, const float* __restrict__ field,
                       const float2* __restrict__ ranges, const float4* __restrict__ bdata,
                       const float* __restrict__ surfZ, const float4* __restrict__ surfN,
@@ -567,7 +571,7 @@ __global__ void __launch_bounds__(128, 8) k_ray(const __grid_constant__ RayParam
   } else {
     const Slab slab = box_hit(ro, rd, volLo, volHi);
     if (slab.hit) {
-      const March m = march(R, field, ranges, bdata, ro, rd, fmaxf(slab.t0, 0.0f) + 1.0e-5f, slab.t1);
+      const March m = march<RANGES>(R, field, ranges, bdata, ro, rd, fmaxf(slab.t0, 0.0f) + 1.0e-5f, slab.t1);
       tHit = m.t;
       hit = m.pos;
     }
@@ -608,7 +612,7 @@ __global__ void __launch_bounds__(128, 8) k_ray(const __grid_constant__ RayParam
       trans = background(R, ro2, refrDir);
     }
     const float tSolid = st.t >= 0.0f ? st.t : 1.0e30f;
-    thick = optical_depth(R, field, ranges, ro2, refrDir, tSolid);
+    thick = optical_depth<RANGES>(R, field, ranges, ro2, refrDir, tSolid);
     trans = {trans.x * fm_exp(-R.absorb[0] * thick), trans.y * fm_exp(-R.absorb[1] * thick),
              trans.z * fm_exp(-R.absorb[2] * thick)};
     col = lerp3(trans, refl, kS);
@@ -678,10 +682,23 @@ void launch_ray(const RayParams& R, const float* field, float2* ranges, const fl
   // With the surface from the mesh the ranges would only shorten the optical depth, which
   // does not pay for the pass that forms them: presets of 8,000 to 500,000 particles at
   // 640 x 480 and 1080p 76-89 / 215-236 us without them, 85-104 / 222-242 us with them.
-  if (R.useSurface != 0) ranges = nullptr;  // the march, which reads them, is not run
-  count_launches(ranges != nullptr ? 2 : 1);
-  if (ranges != nullptr) k_ray_ranges<<<(R.rangeDim[0] * R.rangeDim[1] * R.rangeDim[2] + 3) / 4, tpb, 0, st>>>(R, field, ranges);
-  k_ray<<<grid, tpb, 0, st>>>(R, field, ranges, bodies, surfZ, surfN, image);
+  // Neither does it for a small image of a coarse field. Marching, us a frame alone / three
+  // side by side without and with them, 270 / 486 / 1,683 / 3,468 blocks (dam break of 1,728,
+  // preset of 8,000): 160 x 120 84/23, 104/28, 116/31, 149/43 and 91/25, 107/29, 124/35,
+  // 135/40; 320 x 240 78/23, 109/46, 104/33, 153/59 and 85/25, 110/45, 112/33, 141/53;
+  // 480 x 360 95/34, 140/76, 134/51, 186/93 and 87/27, 129/66, 109/36, 156/75. The form
+  // without ranges is compiled for itself: tested at run time, the pass on the mesh surface
+  // took 3 % longer (250,000 particles at 1080p, three side by side: 172 us, now 166).
+  const int blocks = R.rangeDim[0] * R.rangeDim[1] * R.rangeDim[2];
+  const bool coarse = blocks <= 2000 && (int64_t)R.width * R.height <= 80000;
+  count_launches(1);
+  if (R.useSurface != 0 || coarse) {
+    k_ray<false><<<grid, tpb, 0, st>>>(R, field, nullptr, bodies, surfZ, surfN, image);
+    return;
+  }
+  count_launches(1);
+  k_ray_ranges<<<(blocks + 3) / 4, tpb, 0, st>>>(R, field, ranges);
+  k_ray<true><<<grid, tpb, 0, st>>>(R, field, ranges, bodies, surfZ, surfN, image);
 }
 
 }  // namespace p4a
