@@ -673,6 +673,7 @@ int p4a_tune_get(int32_t kernel, int64_t particles, int32_t* variant);
  *   cell_start          uint32[n_cells+1] out: exclusive scan of cell counts, [n_cells] = n
  *   slot_out            uint32[n] out (may be NULL): sorted position of input i
  *   workspace           device scratch of p4a_grid_sort_workspace_size() bytes
+ * Particle arrays are 16-byte aligned, the workspace 8-byte, the others 4-byte.
  */
 typedef struct p4a_grid {
   float box_min[3];
@@ -688,7 +689,7 @@ size_t p4a_grid_sort_workspace_size(int32_t n, int32_t n_cells);
  *                       *status on `stream` (0 = complete, nonzero = a wait gave
  *                       up); with status == NULL the call waits for `stream` and
  *                       returns P4A_ERR_TIMEOUT when a wait gave up.
- * Returns P4A_ERR_ARG for a NULL grid, n < 0, a dim < 1 or h <= 0, and
+ * Returns P4A_ERR_ARG for a NULL grid, n < 0, a dim < 1, h <= 0 or a misaligned array, and
  * P4A_ERR_CAPACITY when dim[0]*dim[1]*dim[2] exceeds 2^31 - 1 or the workspace is
  * too small; these checks run before any device work. */
 int p4a_grid_sort(const p4a_grid* grid, int32_t n, float dt, float gravity,

@@ -2066,6 +2066,13 @@ int grid_sort_check(const p4a_grid* g, int32_t n, long long maxCells, long long*
   return P4A_OK;
 }
 
+bool grid_sort_aligned(int32_t n, std::initializer_list<const void*> vec4, const uint32_t* cellStart,
+                       const uint32_t* slotOut) {
+  auto at = [](const void* p, uintptr_t bytes) { return (reinterpret_cast<uintptr_t>(p) & (bytes - 1)) == 0; };
+  return at(cellStart, 4) &&
+         (n == 0 || (at(slotOut, 4) && std::all_of(vec4.begin(), vec4.end(), [&](const void* p) { return at(p, 16); })));
+}
+
 int grid_sort_launch(const p4a_grid& g, int32_t n, float dt, float gravity, const float* pos, const float* vel,
                      const uint32_t* body, const float* rest, float* posOut, float* velOut, float* predOut,
                      uint32_t* bodyOut, float* restOut, uint32_t* cellStart, uint32_t* slotOut, uint32_t* key,
@@ -2152,6 +2159,10 @@ int p4a_grid_sort(const p4a_grid* grid, int32_t n, float dt, float gravity, cons
   if (n > 0 && (!pos || !vel || !pos_out || !vel_out || !pred_out)) return P4A_ERR_ARG;
   if ((body && !body_out) || (rest && !rest_out) || !cell_start) return P4A_ERR_ARG;
   if (!workspace || workspace_bytes < p4a_grid_sort_workspace_size(n, nCells)) return P4A_ERR_CAPACITY;
+  if (!grid_sort_aligned(n, {pos, vel, body, rest, pos_out, vel_out, pred_out, body_out, rest_out}, cell_start,
+                         slot_out) ||
+      (reinterpret_cast<uintptr_t>(workspace) & 7) != 0)
+    return P4A_ERR_ARG;
   cudaStream_t st = (cudaStream_t)stream;
   char* w = (char*)workspace;
   const size_t un = (size_t)std::max(1, n);

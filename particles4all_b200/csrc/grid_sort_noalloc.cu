@@ -87,6 +87,9 @@ extern "C" int p4a_grid_sort_noalloc(const p4a_grid* grid, int32_t n, float dt, 
   if ((size_t)n > kMaxN) return P4A_ERR_CAPACITY;
   if (n > 0 && (!pos || !vel || !pos_out || !vel_out || !pred_out)) return P4A_ERR_ARG;
   if ((body && !body_out) || (rest && !rest_out) || !cell_start) return P4A_ERR_ARG;
+  if (!grid_sort_aligned(n, {pos, vel, body, rest, pos_out, vel_out, pred_out, body_out, rest_out}, cell_start,
+                         slot_out))
+    return P4A_ERR_ARG;
   void* base = nullptr;
   rc = scratch_address(&base);
   if (rc != P4A_OK) return rc;

@@ -21,6 +21,7 @@
 #include <stdint.h>
 
 #include <atomic>
+#include <initializer_list>
 
 #include "../../include/p4a.h"
 
@@ -420,6 +421,10 @@ cudaError_t run_grid_sort(const p4a_grid& g, int32_t n, float dt, float gravity,
 extern std::atomic<uint32_t> g_op_spin_limit;
 extern std::atomic<int32_t> g_op_skip_first_tile;
 int grid_sort_check(const p4a_grid* g, int32_t n, long long maxCells, long long* cells);
+// Whether the caller's device arrays have the alignment that the kernels' loads and stores
+// need: a wrong one would be a fault on the device.
+bool grid_sort_aligned(int32_t n, std::initializer_list<const void*> vec4, const uint32_t* cellStart,
+                       const uint32_t* slotOut);
 int grid_sort_launch(const p4a_grid& g, int32_t n, float dt, float gravity, const float* pos, const float* vel,
                      const uint32_t* body, const float* rest, float* posOut, float* velOut, float* predOut,
                      uint32_t* bodyOut, float* restOut, uint32_t* cellStart, uint32_t* slotOut, uint32_t* key,
